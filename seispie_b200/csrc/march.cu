@@ -11,16 +11,33 @@
 //     contiguous range of x rows of one shot.  Every shared-memory access
 //     and every store is a 16-byte vector for four cells; the z neighbours
 //     come from one 8- and one 4-byte load beside it.  The 4th-order x
-//     derivatives of the stress come from register windows of four rows.
+//     derivatives of the stress come from register windows of five rows, and
+//     the arithmetic is packed two cells to an instruction (fma.f32x2 and the
+//     like; each cell's operations and roundings are the scalar kernels').
+//   * Two rows per block barrier: the new velocity of rows r, r+1 goes to a
+//     ring of six rows in shared memory (only rows r-2, r-1 are read across
+//     threads, for D+z, so a row may be overwritten one iteration after its
+//     own column's last use); after the barrier the stress of rows r-2, r-1
+//     follows.  Rows away from a range's ends, the grid's first and last rows
+//     and any source or receiver run a version without a branch, which gives
+//     the compiler one long block to schedule.
 //   * Rows of the state (stress, velocity) stream into a ring of N row slots
 //     in shared memory with untiled bulk copies (cp.async.bulk, one per field
-//     and row, completion on an mbarrier per slot, bounded waits), issued by
-//     one thread N-1 rows ahead of the march.  The model, shared by the shots
-//     and resident in L2, is read with 16-byte loads one row ahead.
-//   * The new velocity of row r goes to an eight-row ring in shared memory;
-//     the stress of row r-2 is updated in the same iteration from that ring
-//     (rows r-3 .. r for D+x, row r-2's neighbours for D+z).  One block
-//     barrier per row.
+//     and row, each issued by its own lane of the last warp, completion on an
+//     mbarrier per slot, bounded waits by every warp for itself).  The model,
+//     shared by the shots and resident in L2, is read with 16-byte loads one
+//     iteration ahead, outside the branches: a load inside one is waited for
+//     where the branches join.
+//   * What bounds it (P-SV 512 x 512, 32 shots): latency with 12 warps per SM
+//     (issue 44 %, DRAM 48 %), not the 470 MB a step has to move at 56 B per
+//     cell (72 us at the measured copy rate; the model and part of the state
+//     come from L2).  One row per barrier, scalar arithmetic and one thread
+//     issuing all copies: 88.7 us and 52.1 M warp instructions per step; this:
+//     69.7 us, 35 M.  1021 x 511, 64 shots: 284 -> 245 us (1.9 GB: 285 us at
+//     the copy rate).  SH 512 x 512, 32 shots: 56 -> 41 us.  256 x 256, one SH
+//     shot: 11.2 -> 5.6 us, where the serial searches of the receiver list
+//     by one thread were most of the step (now a warp tests 32 places at once,
+//     and before the previous step is waited for).
 //   * The rows of all shots form one sequence, split evenly over a grid of
 //     resident CTAs (one pass, no tail wave); a CTA whose range starts in
 //     the middle of a shot recomputes the velocity of the row above its range
@@ -36,8 +53,11 @@
 //     so the per-cell sums are unchanged) and rec_order lists the receivers
 //     by cell.  Each CTA stages the points of its rows in shared-memory
 //     windows and walks them with the march.
+#include <atomic>
 #include <cstdio>
+#include <mutex>
 #include <type_traits>
+#include <vector>
 
 #include "common.cuh"
 #include "stencil.cuh"
@@ -62,11 +82,12 @@ int march_device_status(int clear, int *status) {
 
 constexpr int kPts = 128;        // points (injection entries, receivers) staged per window
 constexpr int kMaxPitch = 1024;  // row length (floats) a CTA can span: 256 threads of 4 columns
-constexpr int kVRing = 5;        // rows of the new-velocity ring (rows s-1 .. s+2 live, plus one for barrier slack)
+constexpr int kVRing = 6;        // rows of the new-velocity ring (r-4 .. r+1)
 
 struct MarchArgs {
     int nx, nz, pitch, nt, it, nrec;
     int rl;                 // shared-memory row length (floats)
+    int nslots;             // row slots of the staging ring
     long long rows_total;   // nshots * nx
     float cx1, cx2, cz1, cz2, dt;
     const float *sig_in[3];
@@ -105,14 +126,19 @@ __host__ __device__ inline MarchLayout march_layout(int nf, int nv, int ninj, in
     return L;
 }
 
-// First index in [lo, hi) whose key is >= v (keys non-decreasing);
-// key(i) = cell[perm ? perm[i] : i].
-__device__ __forceinline__ int lower_bound_cells(const int *cell, const int *perm, int lo, int hi, int v) {
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const int c = cell[perm ? perm[mid] : mid];
-        if (c < v) lo = mid + 1;
-        else hi = mid;
+// First index in [lo, hi) whose key is >= v (keys non-decreasing); key(i) =
+// cell[perm ? perm[i] : i].  Warp-wide: every round tests 32 positions at
+// once, so a list of n points takes log33(n) rounds of dependent loads.
+__device__ __forceinline__ int warp_lower_bound(const int *cell, const int *perm, int lo, int hi, int v) {
+    const int lane = threadIdx.x & 31;
+    while (hi - lo > 0) {
+        const long long n = hi - lo;
+        const int q = lo + (int)(n * (lane + 1) / 33);  // non-decreasing in lane, in [lo, hi)
+        const bool below = cell[perm ? perm[q] : q] < v;
+        const int k = __popc(__ballot_sync(0xffffffffu, below));  // lanes 0 .. k-1 are below
+        const int nlo = k > 0 ? lo + (int)(n * k / 33) + 1 : lo;  // past the last position below
+        hi = k < 32 ? lo + (int)(n * (k + 1) / 33) : hi;          // at the first position not below
+        lo = nlo;
     }
     return lo;
 }
@@ -127,33 +153,73 @@ struct Cursor {
 };
 constexpr int kNone = 0x7fffffff;  // "no further point"
 
-__device__ __forceinline__ void ld4(float (&d)[4], const float *p) {
+// Four adjacent columns as two register pairs: the packed FP32 instructions
+// (one issue slot for two cells) take them as they are loaded.
+struct Q4 {
+    float2 a, b;
+};
+__device__ __forceinline__ Q4 ld4(const float *p) {
     const float4 v = *reinterpret_cast<const float4 *>(p);
-    d[0] = v.x;
-    d[1] = v.y;
-    d[2] = v.z;
-    d[3] = v.w;
+    return Q4{make_float2(v.x, v.y), make_float2(v.z, v.w)};
 }
-__device__ __forceinline__ void st4(float *p, const float (&d)[4]) {
-    *reinterpret_cast<float4 *>(p) = make_float4(d[0], d[1], d[2], d[3]);
-}
-__device__ __forceinline__ void ldg4(float (&d)[4], const float *p) {
+__device__ __forceinline__ Q4 ldg4(const float *p) {
     const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
-    d[0] = v.x;
-    d[1] = v.y;
-    d[2] = v.z;
-    d[3] = v.w;
+    return Q4{make_float2(v.x, v.y), make_float2(v.z, v.w)};
 }
+__device__ __forceinline__ void st4(float *p, const Q4 &q) {
+    *reinterpret_cast<float4 *>(p) = make_float4(q.a.x, q.a.y, q.b.x, q.b.y);
+}
+__device__ __forceinline__ Q4 zero4() { return Q4{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
+// the four values with those whose mask is off set to zero
+__device__ __forceinline__ Q4 keep4(const Q4 &q, const bool (&m)[4]) {
+    return Q4{make_float2(m[0] ? q.a.x : 0.f, m[1] ? q.a.y : 0.f), make_float2(m[2] ? q.b.x : 0.f, m[3] ? q.b.y : 0.f)};
+}
+__device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
 
-template <int MODE, int N>
-__global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_constant__ MarchArgs a) {
+// Finite difference c1 (a - b) - c2 (c - d) of two cells: two differences, the
+// second product, one fused multiply-add -- the operations (and roundings)
+// the scalar kernels' expressions compile to.
+struct Coef {
+    float2 c1, n2;  // c1, -c2
+};
+__device__ __forceinline__ float2 fd2(const Coef &k, float2 a, float2 b, float2 c, float2 d) {
+    const float2 m1 = make_float2(-1.f, -1.f);
+    return __ffma2_rn(k.c1, __ffma2_rn(b, m1, a), __fmul2_rn(k.n2, __ffma2_rn(d, m1, c)));
+}
+__device__ __forceinline__ Q4 fdx(const Coef &k, const Q4 &a, const Q4 &b, const Q4 &c, const Q4 &d) {
+    return Q4{fd2(k, a.a, b.a, c.a, d.a), fd2(k, a.b, b.b, c.b, d.b)};
+}
+// D-z of a row at this thread's columns: taps j, j-1, j+1, j-2 around the
+// centre values c; s points at the row in shared memory
+__device__ __forceinline__ Q4 dzm4(const Coef &k, const float *s, const Q4 &c) {
+    const float2 l = *reinterpret_cast<const float2 *>(s - 2);
+    const float r = s[4];
+    const float2 m0 = make_float2(l.y, c.a.x), m1 = make_float2(c.a.y, c.b.x), m2 = make_float2(c.b.y, r);
+    return Q4{fd2(k, c.a, m0, m1, l), fd2(k, c.b, m1, m2, c.a)};
+}
+// D+z: taps j+1, j, j+2, j-1
+__device__ __forceinline__ Q4 dzp4(const Coef &k, const float *s, const Q4 &c) {
+    const float l = s[-1];
+    const float2 r = *reinterpret_cast<const float2 *>(s + 4);
+    const float2 m0 = make_float2(l, c.a.x), m1 = make_float2(c.a.y, c.b.x), m2 = make_float2(c.b.y, r.x);
+    return Q4{fd2(k, m1, c.a, c.b, m0), fd2(k, m2, c.b, r, m1)};
+}
+__device__ __forceinline__ Q4 add4(const Q4 &x, const Q4 &y) { return Q4{__fadd2_rn(x.a, y.a), __fadd2_rn(x.b, y.b)}; }
+__device__ __forceinline__ Q4 mul4(const Q4 &x, const Q4 &y) { return Q4{__fmul2_rn(x.a, y.a), __fmul2_rn(x.b, y.b)}; }
+__device__ __forceinline__ Q4 fma4(const Q4 &x, const Q4 &y, const Q4 &z) {
+    return Q4{__ffma2_rn(x.a, y.a, z.a), __ffma2_rn(x.b, y.b, z.b)};
+}
+__device__ __forceinline__ float &elem(Q4 &q, int e) { return e == 0 ? q.a.x : e == 1 ? q.a.y : e == 2 ? q.b.x : q.b.y; }
+
+template <int MODE, int WIDE, bool SEG>
+__global__ void __launch_bounds__(WIDE ? 256 : 128, MODE == FWI_SH ? (WIDE ? 2 : 4) : (WIDE ? 1 : 3)) march_kernel(const __grid_constant__ MarchArgs a) {
     using F = Fields<MODE>;
     constexpr int NS = F::NS, NV = F::NV, NF = NS + NV, NINJ = F::NINJ;
     // stress fields with an x register window (D-x) and the one without
     constexpr int FX0 = 0, FX1 = MODE == FWI_SH ? 0 : 2, FZ = 1;
     constexpr int NW = MODE == FWI_SH ? 1 : 2;
     extern __shared__ __align__(128) float smem[];
-    const int RL = a.rl;
+    const int RL = a.rl, N = a.nslots;
     const MarchLayout L = march_layout(NF, NV, NINJ, RL, N);
     int *const i_cell = reinterpret_cast<int *>(smem + L.icell);
     float *const i_val = smem + L.ival;
@@ -163,41 +229,34 @@ __global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_co
     Cursor *const cur_s = reinterpret_cast<Cursor *>(smem + L.cur);
     uint64_t *const full = reinterpret_cast<uint64_t *>(smem + L.bar);
 
-    const int tid = threadIdx.x, j0 = 4 * tid;
+    const int tid = threadIdx.x, j0 = 4 * tid, lane = tid & 31, nwarps = blockDim.x >> 5, warp = tid >> 5;
     const int nx = a.nx, nz = a.nz, pitch = a.pitch, nt = a.nt, it = a.it;
     const bool tin = j0 < pitch;  // this thread's four columns lie in the rows
-    const float cx1 = a.cx1, cx2 = a.cx2, cz1 = a.cz1, cz2 = a.cz2, dt = a.dt;
+    const Coef kx{bc2(a.cx1), bc2(-a.cx2)}, kz{bc2(a.cz1), bc2(-a.cz2)};
+    const Q4 dt4{bc2(a.dt), bc2(a.dt)};
     const uint32_t row_bytes = 4u * (uint32_t)pitch;
     // row buffers start 4 floats into their slot so that columns -4 .. rl-5 are addressable
-    auto ring_row = [&](int slot, int f) -> float * { return smem + (slot * NF + f) * RL + 4; };
-
+    float *const ring0 = smem + 4 + j0;
+    const int slot_len = NF * RL;
 
     grid_dep_trigger();
     if (tid == 0) {
         for (int i = 0; i < N; i++) mbar_init(&full[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    __syncthreads();
-    // the previous step (state rows, and the stress / velocity buffers this
-    // step overwrites) is complete from here on
-    grid_dep_wait();
+    // the field whose rows this lane of the issuing warp streams in, one bulk copy per field and row
+    const bool issuer = warp == nwarps - 1 && lane < NF;
+    const float *my_field = nullptr;
+#pragma unroll
+    for (int f = 0; f < NF; f++)
+        if (lane == f) my_field = f < NS ? a.sig_in[f] : a.vel_in[f < NS ? 0 : f - NS];
 
-    // thread 0: stream row q of the shot at soff into the slot of sequence number sn
-    auto issue = [&](long long soff, int q, int sn) {
-        const int slot = sn % N;
+    // issuing warp, lanes 0 .. NF-1: row q of the shot at soff into ring slot `slot`
+    auto issue = [&](long long soff, int q, int slot) {
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        mbar_expect_tx(&full[slot], NF * row_bytes);
-        const long long o = soff + (long long)q * pitch;
-#pragma unroll
-        for (int f = 0; f < NS; f++) bulk_load(ring_row(slot, f), a.sig_in[f] + o, row_bytes, &full[slot]);
-#pragma unroll
-        for (int c = 0; c < NV; c++) bulk_load(ring_row(slot, NS + c), a.vel_in[c] + o, row_bytes, &full[slot]);
+        if (lane == 0) mbar_expect_tx(&full[slot], NF * row_bytes);
+        bulk_load(smem + slot * slot_len + lane * RL + 4, my_field + soff + (long long)q * pitch, row_bytes, &full[slot]);
     };
-    auto wait_seq = [&](int sn) -> bool { return mbar_wait(&full[sn % N], (uint32_t)((sn / N) & 1)); };
-    // Only warp 0 waits for rows (the others wait at the block barrier that
-    // follows, without issuing); the barrier then makes the landed row
-    // visible to every thread.
-    const bool waiter = tid < 32;
     // per-column masks, fixed for the whole march: D-z (2 <= j < nz-2),
     // D+z (1 <= j < nz-2) and "inside the grid" (j < nz)
     bool zm[4], zp[4], zin[4];
@@ -216,7 +275,25 @@ __global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_co
     const int R = (int)a.rows_total, G = gridDim.x;
     int Lrow = (int)((long long)R * blockIdx.x / G);
     const int Lend = (int)((long long)R * (blockIdx.x + 1) / G);
-    int seq = 0;  // ring sequence number of the next row to issue (same in every thread)
+    int islot = 0;          // ring slot of the next row to issue
+    int wslot = 0;          // ring slot of the next row to wait for
+    uint32_t wphase = 0;    // and the parity of its barrier
+
+    // wait for the next row of the ring (every warp for itself: a row that has
+    // landed costs one test, and no block barrier has to follow)
+    auto wait_next = [&]() -> bool {
+        const bool ok = mbar_try_wait(&full[wslot], wphase) || mbar_wait(&full[wslot], wphase);
+        if (++wslot == N) {
+            wslot = 0;
+            wphase ^= 1;
+        }
+        return ok;
+    };
+    // a wait gave up: record it and let the copies still in flight land
+    auto give_up = [&] {
+        if (tid == 0) atomicExch(&g_march_status, 1);
+        for (int k = 0; k < N; k++) wait_next();
+    };
 
     // stage the window of points starting at c.p (block-wide: every thread
     // calls it with the same cursor, which it updates in place)
@@ -247,9 +324,9 @@ __global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_co
         __syncthreads();
     };
     // after the points of a row: store the cursor into the other buffer of
-    // its list (slow threads may still read the one in use; the row barrier
-    // that follows orders the store before the next use) and return the cell
-    // of the next point, or kNone.  Every thread holds the same cursor.
+    // its list (slow threads may still read the one in use) and return the
+    // cell of the next point, or kNone.  Every thread holds the same cursor;
+    // the barrier orders the store before the next use.
     auto park = [&](Cursor &c, int which, int &buf, bool inj) -> int {
         if (c.p < c.end && c.p - c.w0 >= c.wn) {
             if (inj) load_inj(c);
@@ -258,18 +335,18 @@ __global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_co
         const int nxt = c.p < c.end ? (inj ? i_cell : r_cell)[c.p - c.w0] : kNone;
         buf ^= 1;
         if (tid == 0) cur_s[2 * which + buf] = c;
+        __syncthreads();
         return nxt;
     };
-    // model row `row` at this thread's columns (zero outside the grid)
-    auto ld_model = [&](float (&d)[4], const float *p, int row) {
-        if (tin && row >= 0 && row < nx) {
-            ldg4(d, p + (long long)row * pitch + j0);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; e++) d[e] = 0.f;
-        }
+    // this thread's columns of the model (the first four columns for threads past the row: unused)
+    const long long mcol = tin ? j0 : 0;
+    // model row `row`, or the nearest row of the grid (values outside the grid are not used)
+    auto ld_model = [&](const float *p, int row) -> Q4 {
+        return ldg4(p + (long long)min(max(row, 0), nx - 1) * pitch + mcol);
     };
+    auto wrap = [&](int slot) -> int { return slot >= N ? slot - N : slot; };
 
+    bool first = true;
     while (Lrow < Lend) {
         const int shot = Lrow / nx, a0 = Lrow - shot * nx;
         const int b0 = min(nx, a0 + (Lend - Lrow));
@@ -277,171 +354,151 @@ __global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_co
         const long long soff = (long long)shot * nx * pitch;
         const int va = max(a0 - 1, 0), vb = min(b0 + 2, nx);  // velocity rows computed
         const int qa = max(va - 2, 0), qb = min(vb + 1, nx);  // rows streamed through the ring
-        const int sb = seq - qa;                               // ring sequence number of row q: sb + q
-        seq += qb - qa;
-        int nexti = min(qa + N, qb);
-        if (tid == 0) {
-            for (int q = qa; q < nexti; q++) issue(soff, q, sb + q);
+        int nexti = min(qa + N, qb);                           // next row to issue
+        const int slot_a = islot;                              // ring slot of row qa
+        __syncthreads();  // the previous range's cursors and ring rows are done with
+        if (!first && issuer)
+            for (int q = qa, sl = slot_a; q < nexti; q++, sl = wrap(sl + 1)) issue(soff, q, sl);
+        islot = (slot_a + (nexti - qa)) % N;
+        // the points of this range, found by one warp per list; nothing here depends on the previous
+        // step, so the first range's search runs while that step may still be finishing
+        if (warp == 0) {
             int p0 = 0, p1 = 0;
             if (inj_on) {
                 p0 = a.inj_ptr[shot];
                 p1 = a.inj_ptr[shot + 1];
             }
-            const int i0 = inj_on ? lower_bound_cells(a.inj_cell, nullptr, p0, p1, va * nz) : 0;
-            const int i1 = inj_on ? lower_bound_cells(a.inj_cell, nullptr, p0, p1, vb * nz) : 0;
-            const int r0 = rec_on ? lower_bound_cells(a.rec_cell, a.rec_order, 0, a.nrec, a0 * nz) : 0;
-            const int r1 = rec_on ? lower_bound_cells(a.rec_cell, a.rec_order, 0, a.nrec, b0 * nz) : 0;
-            cur_s[0] = Cursor{i0, i1, i0, 0};
-            cur_s[2] = Cursor{r0, r1, r0, 0};
+            const int i0 = inj_on ? warp_lower_bound(a.inj_cell, nullptr, p0, p1, va * nz) : 0;
+            const int i1 = inj_on ? warp_lower_bound(a.inj_cell, nullptr, i0, p1, vb * nz) : 0;
+            if (lane == 0) cur_s[0] = Cursor{i0, i1, i0, 0};
+        }
+        if (warp == (nwarps > 1 ? 1 : 0)) {
+            const int r0 = rec_on ? warp_lower_bound(a.rec_cell, a.rec_order, 0, a.nrec, a0 * nz) : 0;
+            const int r1 = rec_on ? warp_lower_bound(a.rec_cell, a.rec_order, r0, a.nrec, b0 * nz) : 0;
+            if (lane == 0) cur_s[2] = Cursor{r0, r1, r0, 0};
+        }
+        // model of the rows of the coming iteration: dt/rho and sponge of rows r, r+1, stiffness of rows
+        // r-2, r-1; each is reloaded for the next iteration right after its use
+        Q4 buo[2], bnd[2], ip0[2], ip1[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            buo[k] = ld_model(a.buo, va + k);
+            bnd[k] = ld_model(a.bound, va + k);
+            ip0[k] = ld_model(a.ip[0], va - 2 + k);
+            if (MODE == FWI_PSV) ip1[k] = ld_model(a.ip[1], va - 2 + k);
         }
         __syncthreads();
-        int inj_next, rec_next;  // cell of the next injection entry / receiver, or kNone
+        int inj_next, rec_next;  // row of the next injection entry / receiver, or kNone
         int ib = 0, rb = 0;      // cursor buffers in use
         {
             Cursor c = cur_s[0];
-            inj_next = c.p < c.end ? park(c, 0, ib, true) : kNone;
+            inj_next = c.p < c.end ? park(c, 0, ib, true) / nz : kNone;
             c = cur_s[2];
-            rec_next = c.p < c.end ? park(c, 1, rb, false) : kNone;
+            rec_next = c.p < c.end ? park(c, 1, rb, false) / nz : kNone;
+        }
+        if (first) {
+            // the previous step (state rows, and the stress / velocity buffers this step overwrites) is
+            // complete from here on
+            grid_dep_wait();
+            if (issuer)
+                for (int q = qa, sl = slot_a; q < nexti; q++, sl = wrap(sl + 1)) issue(soff, q, sl);
+            first = false;
         }
 
         bool ok = true;
-        // register windows of four cells: the D-x stress fields at rows
-        // r-2 .. r+1 (SH: sxy; P-SV: sxx, sxz), the other stress field at rows
-        // r-2 .. r (SH: szy; P-SV: szz)
-        float wx[NW][4][4], wz[3][4];
-        // the window rows va-2 .. va must have landed before the first iteration
-        if (waiter)
-            for (int q = qa; q <= va; q++) ok = wait_seq(sb + q) && ok;
-        if (__syncthreads_or(!ok)) goto bail;
+        // Register windows: the D-x stress fields at rows r-2 .. r+2 (SH:
+        // sxy; P-SV: sxx, sxz), the other stress field at rows r-2 .. r+1
+        // (SH: szy; P-SV: szz).
+        Q4 wx[NW][5], wz[4];
+        // rows va-2 .. va must have landed before the first iteration
+        for (int q = qa; q <= va; q++) ok = wait_next() && ok;
+        if (__syncthreads_or(!ok)) return give_up();
+        int scur = slot_a;  // ring slot of row r
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int q = va - 2 + k;
-            if (q >= qa) {
-                const int sl = (sb + q) % N;
-                ld4(wx[0][k], ring_row(sl, FX0) + j0);
-                if (NW > 1) ld4(wx[NW - 1][k], ring_row(sl, FX1) + j0);
-                if (k < 2) ld4(wz[k + 1], ring_row(sl, FZ) + j0);  // rows va-2, va-1 -> wz[1], wz[2]
+        for (int k = 0; k < 2; k++) {
+            if (va - 2 + k >= qa) {
+                const float *s = ring0 + scur * slot_len;
+                wx[0][k] = ld4(s + FX0 * RL);
+                if (NW > 1) wx[NW - 1][k] = ld4(s + FX1 * RL);
+                scur = wrap(scur + 1);
             } else {
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    wx[0][k][e] = wx[NW - 1][k][e] = 0.f;
-                    if (k < 2) wz[k + 1][e] = 0.f;
-                }
+                wx[0][k] = wx[NW - 1][k] = zero4();
             }
+            wz[k] = zero4();
         }
-        // model of the first row: dt/rho and sponge (row va), stiffness (row va-2)
-        float buo[4], bnd[4], ip0[4], ip1[4];
-        ld_model(buo, a.buo, va);
-        ld_model(bnd, a.bound, va);
-        ld_model(ip0, a.ip[0], va - 2);
-        if (MODE == FWI_PSV) ld_model(ip1, a.ip[1], va - 2);
+        {
+            const float *s = ring0 + scur * slot_len;
+            wx[0][2] = ld4(s + FX0 * RL);
+            if (NW > 1) wx[NW - 1][2] = ld4(s + FX1 * RL);
+        }
         // rows above va are consumed once every thread has its window: their
-        // slots take the next rows; then row va+1, which the first iteration
-        // reads, has to land
+        // slots take the next rows
         __syncthreads();
         for (int q = qa; q < va; q++)
             if (nexti < qb) {
-                if (tid == 0) issue(soff, nexti, sb + nexti);
+                if (issuer) issue(soff, nexti, islot);
+                islot = wrap(islot + 1);
                 nexti++;
             }
-        if (waiter && va + 1 < qb) ok = wait_seq(sb + va + 1) && ok;
-        if (__syncthreads_or(!ok)) goto bail;
 
-        // vk: velocity-ring slot of row r
-        for (int r = va, vk = va % kVRing; r < b0 + 2; r++, vk = vk == kVRing - 1 ? 0 : vk + 1) {
-            // next iteration's model values (one row ahead): dt/rho and sponge of row r+1,
-            // stiffness of row r-1
-            float buo_n[4], bnd_n[4], ip0_n[4], ip1_n[4];
-            {
-                const long long m1 = (long long)(r + 1) * pitch + j0, m2 = m1 - 2ll * pitch;
-                const bool ok1 = tin && r + 1 < nx, ok2 = tin && r >= 1 && r - 1 < nx;
+        // this thread's place in row r of the shot (velocity stores; the stress rows lie 2 rows above)
+        long long grow = soff + (long long)va * pitch + j0;
+        // new-velocity ring, three pairs of rows: (r, r+1), (r-2, r-1), (r-4, r-3)
+        float *pa = smem + L.vring + 4 + j0, *pb = pa + 2 * NV * RL, *pc = pb + 2 * NV * RL;
+
+        for (int r = va; r < b0 + 2; r += 2) {
+            const int s1 = wrap(scur + 1), s2 = wrap(scur + 2);
+            if (r + 1 < qb) ok = wait_next() && ok;
+            if (r + 2 < qb) ok = wait_next() && ok;
+            Q4 vn[2][NV];
+            // ---- velocity of rows r, r+1; K: which of the two.  FAST: both rows are this CTA's own, away
+            // from the first and last rows of the grid and without points, so that the row is one stretch
+            // of code without a branch; ZE: this warp holds columns near a z edge (per-column masks).
+            auto velocity = [&](auto k_t, auto fast_t, auto ze_t, const float *scr, const float *snx) {
+                constexpr int K = decltype(k_t)::value;
+                constexpr bool FAST = decltype(fast_t)::value, ZE = decltype(ze_t)::value;
+                const int row = r + K;
+                if (!FAST && row >= vb) {
 #pragma unroll
-                for (int e = 0; e < 4; e++) buo_n[e] = bnd_n[e] = ip0_n[e] = ip1_n[e] = 0.f;
-                if (ok1) {
-                    ldg4(buo_n, a.buo + m1);
-                    ldg4(bnd_n, a.bound + m1);
+                    for (int c = 0; c < NV; c++) {
+                        vn[K][c] = zero4();
+                        st4(pa + (K * NV + c) * RL, vn[K][c]);
+                    }
+                    return;
                 }
-                if (ok2) {
-                    ldg4(ip0_n, a.ip[0] + m2);
-                    if (MODE == FWI_PSV) ldg4(ip1_n, a.ip[1] + m2);
+                if (FAST || row + 1 < qb) {
+                    wx[0][3 + K] = ld4(snx + FX0 * RL);
+                    if (NW > 1) wx[NW - 1][3 + K] = ld4(snx + FX1 * RL);
+                } else {
+                    wx[0][3 + K] = wx[NW - 1][3 + K] = zero4();
                 }
-            }
-            // velocity-ring slots of rows r-3 .. r (row r-3+k in slot vs[k])
-            int vs[4];
+                wz[2 + K] = ld4(scr + FZ * RL);
+                Q4 ds[NV];
+                Q4 zz[NV];  // the z derivative of each component (SH: szy; P-SV: sxz, szz)
+                if constexpr (MODE == FWI_SH) {
+                    zz[0] = dzm4(kz, scr + FZ * RL, wz[2 + K]);
+                } else {
+                    zz[0] = dzm4(kz, scr + FX1 * RL, wx[1][2 + K]);
+                    zz[NV - 1] = dzm4(kz, scr + FZ * RL, wz[2 + K]);
+                }
+                if (ZE) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int q = vk - 3 + k;
-                vs[k] = q < 0 ? q + kVRing : q;
-            }
-            auto vrow = [&](int slot, int c) -> float * { return smem + L.vring + (slot * NV + c) * RL + 4 + j0; };
-            // the z window shifts: wz[0..2] <- rows r-2, r-1, r
+                    for (int c = 0; c < NV; c++) zz[c] = keep4(zz[c], zm);
+                }
+                if (FAST || (row >= 2 && row < nx - 2)) {
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                wz[0][e] = wz[1][e];
-                wz[1][e] = wz[2][e];
-            }
-            float vn[NV][4];
-            const long long grow = soff + (long long)r * pitch + j0;
-            if (r < vb) {
-                // ---- velocity of row r
-                if (r + 1 < qb) {  // landed: waited for before the previous row's barrier
-                    const int sl = (sb + r + 1) % N;
-                    ld4(wx[0][3], ring_row(sl, FX0) + j0);
-                    if (NW > 1) ld4(wx[NW - 1][3], ring_row(sl, FX1) + j0);
+                    for (int c = 0; c < NV; c++)
+                        ds[c] = add4(fdx(kx, wx[c][2 + K], wx[c][1 + K], wx[c][3 + K], wx[c][K]), zz[c]);
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 4; e++) wx[0][3][e] = wx[NW - 1][3][e] = 0.f;
+                    for (int c = 0; c < NV; c++) ds[c] = zz[c];
                 }
-                const int sr = (sb + r) % N;
-                ld4(wz[2], ring_row(sr, FZ) + j0);
-                const bool okx = r >= 2 && r < nx - 2;
-                // D-x of window field w, element e
-                auto dxm = [&](int w, int e) -> float {
-                    return okx ? cx1 * (wx[w][2][e] - wx[w][1][e]) - cx2 * (wx[w][3][e] - wx[w][0][e]) : 0.f;
-                };
-                float ds[NV][4];
-                // the stress divergence; ZE: this warp holds columns near a z edge (per-column masks)
-                auto divergence = [&](auto ze_t) {
-                    constexpr bool ZE = decltype(ze_t)::value;
-                    // D-z of stress field f at row r, element e, from columns j0-2 .. j0+4:
-                    // x[i] = column j0-2+i, with the centre taken from `cen`
-                    auto dzm_row = [&](int f, const float (&cen)[4], float (&out)[4]) {
-                        const float *s = ring_row(sr, f) + j0;
-                        const float2 l2 = *reinterpret_cast<const float2 *>(s - 2);
-                        const float rr = s[4];
-                        const float x[7] = {l2.x, l2.y, cen[0], cen[1], cen[2], cen[3], rr};
+                // sources of the row, summed per cell in entry order (stf_dsy / stf_dsxz, solver.py:78-93)
+                if (!FAST && inj_next <= row) {
+                    const int lo = row * nz, hi = lo + nz;
+                    Q4 acc[NINJ];
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float d = cz1 * (x[e + 2] - x[e + 1]) - cz2 * (x[e + 3] - x[e]);
-                            out[e] = (!ZE || zm[e]) ? d : 0.f;
-                        }
-                    };
-                    if constexpr (MODE == FWI_SH) {
-                        float zz[4];
-                        dzm_row(1, wz[2], zz);
-#pragma unroll
-                        for (int e = 0; e < 4; e++) ds[0][e] = dxm(0, e) + zz[e];
-                    } else {
-                        float zxz[4], zzz[4];
-                        dzm_row(2, wx[1][2], zxz);
-                        dzm_row(1, wz[2], zzz);
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            ds[0][e] = dxm(0, e) + zxz[e];
-                            ds[1][e] = dxm(1, e) + zzz[e];
-                        }
-                    }
-                };
-                if (zedge) divergence(std::true_type{});
-                else divergence(std::false_type{});
-                // sources of row r, summed per cell in entry order (stf_dsy / stf_dsxz, solver.py:78-93)
-                if (inj_next < (r + 1) * nz) {
-                    const int lo = r * nz, hi = lo + nz;
-                    float acc[NINJ][4];
-#pragma unroll
-                    for (int q = 0; q < NINJ; q++)
-#pragma unroll
-                        for (int e = 0; e < 4; e++) acc[q][e] = 0.f;
+                    for (int q = 0; q < NINJ; q++) acc[q] = zero4();
                     Cursor c = cur_s[ib];
                     while (c.p < c.end) {
                         if (c.p - c.w0 >= c.wn) load_inj(c);
@@ -452,41 +509,33 @@ __global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_co
                         for (int e = 0; e < 4; e++)
                             if (off == e) {
 #pragma unroll
-                                for (int q = 0; q < NINJ; q++) acc[q][e] += i_val[q * kPts + k];
+                                for (int q = 0; q < NINJ; q++) elem(acc[q], e) += i_val[q * kPts + k];
                             }
                         c.p++;
                     }
-                    inj_next = park(c, 0, ib, true);
+                    const int nxt = park(c, 0, ib, true);
+                    inj_next = nxt == kNone ? kNone : nxt / nz;
 #pragma unroll
-                    for (int q = 0; q < NV; q++)
-#pragma unroll
-                        for (int e = 0; e < 4; e++) ds[q][e] += acc[q][e];
+                    for (int q = 0; q < NV; q++) ds[q] = add4(ds[q], acc[q]);
                 }
-                const bool own = r >= a0 && r < b0 && tin;
-                auto velocity = [&](auto ze_t) {
-                    constexpr bool ZE = decltype(ze_t)::value;
+                const bool own = (FAST || (row >= a0 && row < b0)) && (!ZE || tin);
 #pragma unroll
-                    for (int c = 0; c < NV; c++) {
-                        float vold[4];
-                        ld4(vold, ring_row(sr, NS + c) + j0);
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float v = bnd[e] * (vold[e] + ds[c][e] * buo[e]);
-                            vn[c][e] = (!ZE || zin[e]) ? v : 0.f;  // padding columns stay zero
-                            if (ZE && !zin[e]) ds[c][e] = 0.f;
-                        }
-                        st4(vrow(vs[3], c), vn[c]);
-                        if (own) {
-                            st4(a.vel_out[c] + grow, vn[c]);
-                            if (a.seg_ds[c]) st4(a.seg_ds[c] + grow, ds[c]);
-                        }
+                for (int c = 0; c < NV; c++) {
+                    const Q4 vold = ld4(scr + (NS + c) * RL);
+                    vn[K][c] = mul4(bnd[K], fma4(ds[c], buo[K], vold));
+                    if (ZE) {  // padding columns stay zero
+                        vn[K][c] = keep4(vn[K][c], zin);
+                        ds[c] = keep4(ds[c], zin);
                     }
-                };
-                if (zedge) velocity(std::true_type{});
-                else velocity(std::false_type{});
-                // receivers of row r record the new velocity (save_obs, solver.py:151-156)
-                if (rec_next < (r + 1) * nz) {
-                    const int lo = r * nz, hi = lo + nz;
+                    st4(pa + (K * NV + c) * RL, vn[K][c]);
+                    if (own) {
+                        st4(a.vel_out[c] + grow + K * pitch, vn[K][c]);
+                        if (SEG && a.seg_ds[c]) st4(a.seg_ds[c] + grow + K * pitch, ds[c]);
+                    }
+                }
+                // receivers of the row record the new velocity (save_obs, solver.py:151-156)
+                if (!FAST && rec_next <= row) {
+                    const int lo = row * nz, hi = lo + nz;
                     Cursor c = cur_s[2 + rb];
                     while (c.p < c.end) {
                         if (c.p - c.w0 >= c.wn) load_rec(c);
@@ -500,121 +549,142 @@ __global__ void __launch_bounds__(kMaxPitch / 4, 2) march_kernel(const __grid_co
                                 if (off == e) {
 #pragma unroll
                                     for (int q = 0; q < NV; q++)
-                                        if (a.obs[q]) a.obs[q][o] = vn[q][e];
+                                        if (a.obs[q]) a.obs[q][o] = elem(vn[K][q], e);
                                 }
                         }
                         c.p++;
                     }
-                    rec_next = park(c, 1, rb, false);
+                    const int nxt = park(c, 1, rb, false);
+                    rec_next = nxt == kNone ? kNone : nxt / nz;
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < NV; c++) {
-#pragma unroll
-                    for (int e = 0; e < 4; e++) vn[c][e] = 0.f;
-                    st4(vrow(vs[3], c), vn[c]);
-                }
-            }
-            // the next iteration reads row r+2: warp 0 waits for it before the barrier
-            if (waiter && r + 2 < qb && r + 2 < vb + 1) ok = wait_seq(sb + r + 2) && ok;
-            if (__syncthreads_or(!ok)) goto bail;
-            // row r is consumed: its slot takes row r + N
-            if (nexti < qb) {
-                if (tid == 0) issue(soff, nexti, sb + nexti);
-                nexti++;
-            }
-
-            // ---- stress of row s = r - 2 (add_sy / add_sxz, solver.py:128-149)
-            const int s = r - 2;
-            auto stress = [&](auto ze_t) {
-                constexpr bool ZE = decltype(ze_t)::value;
-                const bool okx = s >= 1 && s < nx - 2;
-                const long long gs = soff + (long long)s * pitch + j0;
-                float ex[NV][4], ez[NV][4];
-#pragma unroll
-                for (int c = 0; c < NV; c++) {
-                    // rows s-1 .. s+2 of the new velocity, and row s's z neighbours:
-                    // y[i] = column j0-1+i of row s
-                    float v0[4], v1[4], v2[4], v3[4];
-                    ld4(v0, vrow(vs[0], c));
-                    ld4(v1, vrow(vs[1], c));
-                    ld4(v2, vrow(vs[2], c));
-                    ld4(v3, vrow(vs[3], c));
-                    const float *vsr = vrow(vs[1], c);
-                    const float l1 = vsr[-1];
-                    const float2 r2 = *reinterpret_cast<const float2 *>(vsr + 4);
-                    const float y[7] = {l1, v1[0], v1[1], v1[2], v1[3], r2.x, r2.y};
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        ex[c][e] = okx ? cx1 * (v2[e] - v1[e]) - cx2 * (v3[e] - v0[e]) : 0.f;
-                        const float d = cz1 * (y[e + 2] - y[e + 1]) - cz2 * (y[e + 3] - y[e]);
-                        ez[c][e] = (!ZE || zp[e]) ? d : 0.f;
-                    }
-                }
-                if constexpr (MODE == FWI_SH) {
-                    float o0[4], o1[4];
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float dm = dt * ip0[e], exy = ex[0][e], ezy = ez[0][e];
-                        const bool in = !ZE || zin[e];  // padding columns stay zero
-                        o0[e] = in ? wx[0][0][e] + dm * exy : 0.f;
-                        o1[e] = in ? wz[0][e] + dm * ezy : 0.f;
-                    }
-                    st4(a.sig_out[0] + gs, o0);
-                    st4(a.sig_out[1] + gs, o1);
-                    if (a.seg_e[0]) {
-                        st4(a.seg_e[0] + gs, ex[0]);
-                        st4(a.seg_e[1] + gs, ez[0]);
+            };
+            {
+                const float *c0 = ring0 + scur * slot_len, *c1 = ring0 + s1 * slot_len, *c2 = ring0 + s2 * slot_len;
+                const std::integral_constant<int, 0> k0{};
+                const std::integral_constant<int, 1> k1{};
+                const std::true_type yes{};
+                const std::false_type no{};
+                if (r >= max(a0, 2) && r + 1 < min(b0, nx - 2) && min(inj_next, rec_next) > r + 1) {
+                    if (zedge) {
+                        velocity(k0, yes, yes, c0, c1);
+                        velocity(k1, yes, yes, c1, c2);
+                    } else {
+                        velocity(k0, yes, no, c0, c1);
+                        velocity(k1, yes, no, c1, c2);
                     }
                 } else {
-                    float o0[4], o1[4], o2[4], sh[4];
+                    velocity(k0, no, yes, c0, c1);
+                    velocity(k1, no, yes, c1, c2);
+                }
+            }
+            // the next iteration's dt/rho and sponge, in flight during the barrier and the stress half (loaded
+            // here and not in the branches above, whose join would wait for them)
 #pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float lam = ip0[e], mu = ip1[e];
-                        const float vxx = ex[0][e], vxz = ez[0][e], vzx = ex[1][e], vzz = ez[1][e];
-                        const float l2m = lam + 2.f * mu, shear = vxz + vzx;
-                        const bool in = !ZE || zin[e];  // padding columns stay zero
-                        o0[e] = in ? wx[0][0][e] + dt * (l2m * vxx + lam * vzz) : 0.f;
-                        o1[e] = in ? wz[0][e] + dt * (l2m * vzz + lam * vxx) : 0.f;
-                        o2[e] = in ? wx[1][0][e] + dt * (mu * shear) : 0.f;
-                        sh[e] = in ? shear : 0.f;
+            for (int k = 0; k < 2; k++) {
+                buo[k] = ld_model(a.buo, r + 2 + k);
+                bnd[k] = ld_model(a.bound, r + 2 + k);
+            }
+            if (__syncthreads_or(!ok)) return give_up();
+            // rows r and r+1 are consumed: their slots take rows r + N, r + N + 1
+            scur = s2;
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                if (nexti < qb) {
+                    if (issuer) issue(soff, nexti, islot);
+                    islot = wrap(islot + 1);
+                    nexti++;
+                }
+
+            // ---- stress of rows r-2, r-1 (add_sy / add_sxz, solver.py:128-149)
+            Q4 vw[NV][3];  // new velocity of rows r-3, r-2, r-1
+#pragma unroll
+            for (int c = 0; c < NV; c++) {
+                vw[c][0] = ld4(pc + (NV + c) * RL);
+                vw[c][1] = ld4(pb + c * RL);
+                vw[c][2] = ld4(pb + (NV + c) * RL);
+            }
+            auto stress = [&](auto k_t, auto fast_t, auto ze_t) {
+                constexpr int K = decltype(k_t)::value;
+                constexpr bool FAST = decltype(fast_t)::value, ZE = decltype(ze_t)::value;
+                const int s = r - 2 + K;
+                if ((FAST || (s >= a0 && s < b0)) && (!ZE || tin)) {
+                    Q4 ex[NV], ez[NV];
+#pragma unroll
+                    for (int c = 0; c < NV; c++) {
+                        const Q4 &v0 = vw[c][K], &v1 = vw[c][1 + K];
+                        const Q4 &v2 = K == 0 ? vw[c][2] : vn[0][c], &v3 = vn[K][c];
+                        ez[c] = dzp4(kz, pb + (K * NV + c) * RL, v1);
+                        if (ZE) ez[c] = keep4(ez[c], zp);
+                        if (FAST || (s >= 1 && s < nx - 2)) ex[c] = fdx(kx, v2, v1, v3, v0);
+                        else ex[c] = zero4();
                     }
-                    st4(a.sig_out[0] + gs, o0);
-                    st4(a.sig_out[1] + gs, o1);
-                    st4(a.sig_out[2] + gs, o2);
-                    if (a.seg_e[0]) {
+                    Q4 o[NS], shear = zero4();
+                    if constexpr (MODE == FWI_SH) {
+                        const Q4 dm = mul4(dt4, ip0[K]);
+                        o[0] = fma4(dm, ex[0], wx[0][K]);
+                        o[1] = fma4(dm, ez[0], wz[K]);
+                    } else {
+                        shear = add4(ez[0], ex[NV - 1]);
+                        const Q4 two{bc2(2.f), bc2(2.f)};
+                        const Q4 l2m = fma4(two, ip1[K], ip0[K]);
+                        o[0] = fma4(dt4, fma4(l2m, ex[0], mul4(ip0[K], ez[NV - 1])), wx[0][K]);
+                        o[1] = fma4(dt4, fma4(ip0[K], ex[0], mul4(l2m, ez[NV - 1])), wz[K]);
+                        o[NS - 1] = fma4(dt4, mul4(ip1[K], shear), wx[NW - 1][K]);
+                    }
+                    if (ZE) {  // padding columns stay zero
+#pragma unroll
+                        for (int f = 0; f < NS; f++) o[f] = keep4(o[f], zin);
+                        if (SEG && MODE == FWI_PSV) shear = keep4(shear, zin);
+                    }
+                    const long long gs = grow + (K - 2) * pitch;
+#pragma unroll
+                    for (int f = 0; f < NS; f++) st4(a.sig_out[f] + gs, o[f]);
+                    if (SEG && a.seg_e[0]) {
                         st4(a.seg_e[0] + gs, ex[0]);
-                        st4(a.seg_e[1] + gs, ez[1]);
-                        st4(a.seg_e[2] + gs, sh);
+                        st4(a.seg_e[1] + gs, ez[NV - 1]);
+                        if (MODE == FWI_PSV) st4(a.seg_e[NS - 1] + gs, shear);
                     }
                 }
             };
-            if (s >= a0 && s < b0 && tin) {
-                if (zedge) stress(std::true_type{});
-                else stress(std::false_type{});
-            }
-#pragma unroll
-            for (int w = 0; w < NW; w++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    wx[w][0][e] = wx[w][1][e];
-                    wx[w][1][e] = wx[w][2][e];
-                    wx[w][2][e] = wx[w][3][e];
+            {
+                const std::integral_constant<int, 0> k0{};
+                const std::integral_constant<int, 1> k1{};
+                const std::true_type yes{};
+                const std::false_type no{};
+                if (r - 2 >= max(a0, 1) && r - 1 < min(b0, nx - 2)) {
+                    if (zedge) {
+                        stress(k0, yes, yes);
+                        stress(k1, yes, yes);
+                    } else {
+                        stress(k0, yes, no);
+                        stress(k1, yes, no);
+                    }
+                } else {
+                    stress(k0, no, yes);
+                    stress(k1, no, yes);
                 }
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                buo[e] = buo_n[e];
-                bnd[e] = bnd_n[e];
-                ip0[e] = ip0_n[e];
-                if (MODE == FWI_PSV) ip1[e] = ip1_n[e];
             }
+            // and its stiffness, in flight during the next velocity half
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                ip0[k] = ld_model(a.ip[0], r + k);
+                if (MODE == FWI_PSV) ip1[k] = ld_model(a.ip[1], r + k);
+            }
+            // the windows move down two rows
+#pragma unroll
+            for (int w = 0; w < NW; w++) {
+                wx[w][0] = wx[w][2];
+                wx[w][1] = wx[w][3];
+                wx[w][2] = wx[w][4];
+            }
+            wz[0] = wz[2];
+            wz[1] = wz[3];
+            float *const t = pc;
+            pc = pb;
+            pb = pa;
+            pa = t;
+            grow += 2 * pitch;
         }
-        continue;
-    bail:
-        // a wait gave up: let the copies still in flight land, then stop
-        if (tid == 0) atomicExch(&g_march_status, 1);
-        for (int q = max(qa, nexti - N); q < nexti; q++) wait_seq(sb + q);
-        return;
     }
 }
 
@@ -647,87 +717,97 @@ bool march_supported(const fwi_batch *b) {
     return (b->mode == FWI_SH || b->mode == FWI_PSV) && b->pitch <= kMaxPitch;
 }
 
-template <int MODE, int N>
-static int march_occupancy(int nthr, size_t bytes, int *occ) {
-    cudaError_t e = cudaFuncSetAttribute(march_kernel<MODE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, march_kernel<MODE, N>, nthr, bytes);
-    if (e != cudaSuccess) return set_error(FWI_ECUDA, "march_kernel occupancy: %s", cudaGetErrorString(e));
-    return 0;
-}
-
-template <int MODE>
-static int march_occupancy_n(int n, int nthr, size_t bytes, int *occ) {
-    switch (n) {
-        case 3: return march_occupancy<MODE, 3>(nthr, bytes, occ);
-        case 4: return march_occupancy<MODE, 4>(nthr, bytes, occ);
-        case 6: return march_occupancy<MODE, 6>(nthr, bytes, occ);
-        default: return march_occupancy<MODE, 8>(nthr, bytes, occ);
-    }
-}
+constexpr size_t kMaxSmem = 227 * 1024;
 
 // Ring depth and resident CTAs per SM for a launch shape: the requested
 // depth, or the one with the most resident CTAs (shared memory and
-// registers both counted), the deepest among those.  Cached per shape.
-template <int MODE>
-static int march_choose(int nthr, int rl, int want, int *n_out, size_t *bytes_out, int *occ_out) {
-    struct Entry {
-        int nthr, rl, want, n, occ;
-        size_t bytes;
-    };
-    static Entry cache[16];
-    static int ncache = 0;
-    for (int i = 0; i < ncache; i++)
-        if (cache[i].nthr == nthr && cache[i].rl == rl && cache[i].want == want) {
-            *n_out = cache[i].n;
-            *bytes_out = cache[i].bytes;
-            *occ_out = cache[i].occ;
+// registers both counted), the deepest among those.  Made once per shape;
+// the kernel's dynamic shared memory limit is the SM's throughout, so that a
+// shape's plan does not depend on which other shapes have run.
+struct MarchPlan {
+    int nthr, rl, want, n, occ;
+    size_t bytes;
+};
+
+template <int MODE, int WIDE, bool SEG>
+static int march_choose(int nthr, int rl, int want, MarchPlan *out) {
+    static std::mutex lock;
+    static std::vector<MarchPlan> plans;
+    const auto kernel = march_kernel<MODE, WIDE, SEG>;
+    std::lock_guard<std::mutex> hold(lock);
+    if (plans.empty()) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+        if (e != cudaSuccess) return set_error(FWI_ECUDA, "march_kernel shared memory: %s", cudaGetErrorString(e));
+    }
+    for (const MarchPlan &p : plans)
+        if (p.nthr == nthr && p.rl == rl && p.want == want) {
+            *out = p;
             return 0;
         }
-    int best = 0, best_occ = 0;
-    size_t best_bytes = 0;
+    MarchPlan best{nthr, rl, want, 0, 0, 0};
     for (int n : {3, 4, 6, 8}) {
         if (want && n != want) continue;
         const size_t b = march_bytes(MODE, rl, n);
-        if (b > (size_t)227 * 1024) continue;
+        if (b > kMaxSmem) continue;
         int occ = 0;
-        const int rc = march_occupancy_n<MODE>(n, nthr, b, &occ);
-        if (rc) return rc;
-        if (occ >= 1 && occ >= best_occ) {
-            best = n;
-            best_occ = occ;
-            best_bytes = b;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, nthr, b);
+        if (e != cudaSuccess) return set_error(FWI_ECUDA, "march_kernel occupancy: %s", cudaGetErrorString(e));
+        if (occ >= 1 && occ >= best.occ) {
+            best.n = n;
+            best.occ = occ;
+            best.bytes = b;
         }
     }
-    if (!best) return set_error(FWI_ERANGE, "row-marching step: rows of %d floats do not fit an SM", rl - 8);
-    if (ncache < 16) cache[ncache++] = Entry{nthr, rl, want, best, best_occ, best_bytes};
-    *n_out = best;
-    *bytes_out = best_bytes;
-    *occ_out = best_occ;
+    if (!best.n) return set_error(FWI_ERANGE, "row-marching step: rows of %d floats do not fit an SM", rl - 8);
+    plans.push_back(best);
+    *out = best;
     return 0;
 }
 
-template <int MODE, int N>
-static int launch_march_mode(const MarchArgs &a, int nthr, size_t bytes, int occ, bool pdl, cudaStream_t st) {
-    static int sms = 0;
-    if (!sms) {
+static int sm_count() {
+    static std::atomic<int> sms{0};
+    int n = sms.load(std::memory_order_relaxed);
+    if (!n) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-            sms = 148;
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+            n = 148;
+        sms.store(n, std::memory_order_relaxed);
     }
-    const long long grid = a.rows_total < (long long)sms * occ ? a.rows_total : (long long)sms * occ;
+    return n;
+}
+
+template <int MODE, int WIDE, bool SEG>
+static int launch_march_mode(MarchArgs &a, int nthr, int want, int cap, bool pdl, cudaStream_t st) {
+    MarchPlan p;
+    const int rc = march_choose<MODE, WIDE, SEG>(nthr, a.rl, want, &p);
+    if (rc) return rc;
+    a.nslots = p.n;
+    const int occ = cap > 0 && cap < p.occ ? cap : p.occ;
+    const long long slots = (long long)sm_count() * occ;
+    const long long grid = a.rows_total < slots ? a.rows_total : slots;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(nthr, 1, 1);
-    cfg.dynamicSmemBytes = bytes;
+    cfg.dynamicSmemBytes = p.bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     set_pdl_attr(attr[0], true);
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, march_kernel<MODE, N>, a);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, march_kernel<MODE, WIDE, SEG>, a);
     if (e != cudaSuccess) return set_error(FWI_ECUDA, "march_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("march_kernel");
+}
+
+template <int MODE>
+static int launch_march_any(MarchArgs &a, int nthr, int want, int cap, bool pdl, cudaStream_t st) {
+    const bool seg = a.seg_e[0] || a.seg_ds[0] || a.seg_ds[1];
+    if (nthr > 128)
+        return seg ? launch_march_mode<MODE, 1, true>(a, nthr, want, cap, pdl, st)
+                   : launch_march_mode<MODE, 1, false>(a, nthr, want, cap, pdl, st);
+    return seg ? launch_march_mode<MODE, 0, true>(a, nthr, want, cap, pdl, st)
+               : launch_march_mode<MODE, 0, false>(a, nthr, want, cap, pdl, st);
 }
 
 int launch_march(const fwi_batch *b, int it, bool pdl, cudaStream_t st) {
@@ -779,26 +859,8 @@ int launch_march(const fwi_batch *b, int it, bool pdl, cudaStream_t st) {
     // four columns per thread, whole warps
     const int nthr = ((b->pitch / 4 + 31) / 32) * 32;
     a.rl = 4 * nthr + 8;
-    size_t bytes = 0;
-    int n = 0, occ = 0;
-    int rc = mode == FWI_SH ? march_choose<FWI_SH>(nthr, a.rl, b->ring, &n, &bytes, &occ)
-                            : march_choose<FWI_PSV>(nthr, a.rl, b->ring, &n, &bytes, &occ);
-    if (rc) return rc;
-    if (b->ctas_per_sm > 0 && b->ctas_per_sm < occ) occ = b->ctas_per_sm;
-    if (mode == FWI_SH) {
-        switch (n) {
-            case 3: return launch_march_mode<FWI_SH, 3>(a, nthr, bytes, occ, pdl, st);
-            case 4: return launch_march_mode<FWI_SH, 4>(a, nthr, bytes, occ, pdl, st);
-            case 6: return launch_march_mode<FWI_SH, 6>(a, nthr, bytes, occ, pdl, st);
-            default: return launch_march_mode<FWI_SH, 8>(a, nthr, bytes, occ, pdl, st);
-        }
-    }
-    switch (n) {
-        case 3: return launch_march_mode<FWI_PSV, 3>(a, nthr, bytes, occ, pdl, st);
-        case 4: return launch_march_mode<FWI_PSV, 4>(a, nthr, bytes, occ, pdl, st);
-        case 6: return launch_march_mode<FWI_PSV, 6>(a, nthr, bytes, occ, pdl, st);
-        default: return launch_march_mode<FWI_PSV, 8>(a, nthr, bytes, occ, pdl, st);
-    }
+    return mode == FWI_SH ? launch_march_any<FWI_SH>(a, nthr, b->ring, b->ctas_per_sm, pdl, st)
+                          : launch_march_any<FWI_PSV>(a, nthr, b->ring, b->ctas_per_sm, pdl, st);
 }
 
 // A bounded wait on an mbarrier that nothing ever completes: the wait runs
