@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <atomic>
 #include <cstring>
+#include <memory>
 
 #include "common.cuh"
 
@@ -32,10 +33,16 @@ int check_launch(const char *what) {
 }
 
 // defined in step.cu / aux.cu
+struct StepPlan;  // tensor maps kept over a time loop
+StepPlan *make_step_plan();
+void free_step_plan(StepPlan *p);
+struct AdjPlan;
+AdjPlan *make_adj_plan();
+void free_adj_plan(AdjPlan *p);
 int launch_step(const fwi_batch *b, int adjoint, int it, bool snap_u_next, int snap_u_slot, bool snap_v,
-                int snap_v_slot, cudaStream_t st);
+                int snap_v_slot, bool pdl, StepPlan *plan, cudaStream_t st);
 int launch_interaction(const fwi_batch *b, int isae, cudaStream_t st);
-int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, cudaStream_t st);
+int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, AdjPlan *plan, cudaStream_t st);
 int launch_march(const fwi_batch *b, int it, bool pdl, cudaStream_t st);
 bool march_supported(const fwi_batch *b);
 int launch_displacement_traces(float *obs, long long ntr, int nt, int it0, int n, double dt, cudaStream_t st);
@@ -270,6 +277,8 @@ int fwi_run(fwi_batch *b, int adjoint, int it0, int nsteps, void *stream) {
             }
         }
     }
+    const std::unique_ptr<StepPlan, void (*)(StepPlan *)> plan(make_step_plan(), free_step_plan);
+    REQUIRE(plan, "fwi_run: out of host memory");
     for (int it = it0; it < it0 + nsteps; it++) {
         bool su = false, sv = false;
         int sus = 0, svs = 0;
@@ -283,7 +292,7 @@ int fwi_run(fwi_batch *b, int adjoint, int it0, int nsteps, void *stream) {
                 sv = svs >= 0 && svs < nsa;
             }
         }
-        rc = launch_step(b, adjoint, it, su, sus, sv, svs, st);
+        rc = launch_step(b, adjoint, it, su, sus, sv, svs, b->step_overlap != 0 && it > it0, plan.get(), st);
         if (rc) return rc;
         b->cur ^= 1;
         if (adjoint && it % sae == 0) {
@@ -321,8 +330,10 @@ int fwi_run_transposed(fwi_batch *b, int it_hi, int nsteps, void *stream) {
     cudaStream_t st = (cudaStream_t)stream;
     // every launch after the first follows a transposed step of this loop directly
     const bool pdl = b->step_overlap != 0;
+    const std::unique_ptr<AdjPlan, void (*)(AdjPlan *)> plan(make_adj_plan(), free_adj_plan);
+    REQUIRE(plan, "fwi_run_transposed: out of host memory");
     for (int it = it_hi - 1; it >= it_hi - nsteps; it--) {
-        rc = launch_adjoint_step(b, it, pdl && it < it_hi - 1, st);
+        rc = launch_adjoint_step(b, it, pdl && it < it_hi - 1, plan.get(), st);
         if (rc) return rc;
         b->cur ^= 1;
     }

@@ -40,6 +40,7 @@
 #include <type_traits>
 
 #include <cstdio>
+#include <new>
 
 #include "common.cuh"
 #include "stencil.cuh"
@@ -536,6 +537,10 @@ __device__ __forceinline__ void rw_body(const StepArgs &a, const TmaMaps &maps, 
     const int nx = a.nx, nz = a.nz, pitch = a.pitch;
     const long long soff = (long long)shot * nx * pitch;
     bool has_inj;
+    // the next step may be scheduled; the previous one (the state this step reads, and the buffers it
+    // overwrites) is complete from here on
+    grid_dep_trigger();
+    grid_dep_wait();
     if constexpr (TMA) {
         const int r = prologue_tma<MODE, TX, TZ>(a, maps, sm, reinterpret_cast<uint64_t *>(smem + T::BAR_OFF), x0,
                                                  z0, shot);
@@ -711,12 +716,24 @@ static int build_maps(const StepArgs &a, int nshots, TmaMaps &m) {
     return rc;
 }
 
+// Tensor maps of a time loop, encoded by its first launch on each half of the
+// ping-pong pairs and kept for the loop's other launches: encoding the ten to
+// nineteen maps of a step takes the host about as long as a small grid's step
+// takes the GPU.  With early launches (grid_dep_trigger) beside it: spin 500 x
+// 412, 8 shots 48.5 -> 46.5 us per step; spin gradient 320 x 208, 4 shots,
+// 100 steps 7.98 -> 7.49 ms.
+struct StepPlan {
+    TmaMaps maps[2];
+    bool have[2];
+};
+StepPlan *make_step_plan() { return new (std::nothrow) StepPlan(); }
+void free_step_plan(StepPlan *p) { delete p; }
+
 // kind: 0 generic mapping, 1 register window (cp.async), 2 register window (TMA)
 template <int MODE, int TX, int TZ, int KIND>
-static int launch_tile(const StepArgs &a, int nshots, cudaStream_t st) {
+static int launch_tile(const StepArgs &a, int nshots, int cur, bool pdl, StepPlan *plan, cudaStream_t st) {
     using T = Tile<MODE, TX, TZ>;
     static bool attr_set = false;
-    static TmaMaps none;  // unused by the cp.async variants
     if constexpr (KIND == 0) {
         if (!attr_set) {
             cudaError_t e = cudaFuncSetAttribute(step_kernel<MODE, TX, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -735,34 +752,42 @@ static int launch_tile(const StepArgs &a, int nshots, cudaStream_t st) {
             if (e != cudaSuccess) return set_error(FWI_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
             attr_set = true;
         }
-        const TmaMaps *maps = &none;
-        TmaMaps built;
-        if constexpr (TMA) {
-            int rc = build_maps<MODE, TX, TZ>(a, nshots, built);
+        TmaMaps &maps = plan->maps[cur];  // unused by the cp.async variants
+        if (TMA && !plan->have[cur]) {
+            const int rc = build_maps<MODE, TX, TZ>(a, nshots, maps);
             if (rc) return rc;
-            maps = &built;
+            plan->have[cur] = true;
         }
-        dim3 grid((a.nz + TZ - 1) / TZ, (a.nx + TX - 1) / TX, nshots);
-        step_kernel_rw<MODE, TX, TMA><<<grid, kThreads, T::bytes, st>>>(a, *maps);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((a.nz + TZ - 1) / TZ, (a.nx + TX - 1) / TX, nshots);
+        cfg.blockDim = dim3(kThreads, 1, 1);
+        cfg.dynamicSmemBytes = T::bytes;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        set_pdl_attr(attr[0], true);
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl ? 1 : 0;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, step_kernel_rw<MODE, TX, TMA>, a, maps);
+        if (e != cudaSuccess) return set_error(FWI_ECUDA, "step_kernel launch: %s", cudaGetErrorString(e));
     }
     return check_launch("step_kernel");
 }
 
 template <int MODE>
-static int launch_mode(const StepArgs &a, int nshots, int tile, cudaStream_t st) {
+static int launch_mode(const StepArgs &a, int nshots, int tile, int cur, bool pdl, StepPlan *plan, cudaStream_t st) {
     switch (tile) {
-        case 0: return launch_tile<MODE, 32, 32, 2>(a, nshots, st);
-        case 1: return launch_tile<MODE, 32, 32, 0>(a, nshots, st);
-        case 2: return launch_tile<MODE, 16, 64, 0>(a, nshots, st);
-        case 3: return launch_tile<MODE, 16, 32, 0>(a, nshots, st);
-        case 4: return launch_tile<MODE, 64, 32, 0>(a, nshots, st);
-        case 5: return launch_tile<MODE, 8, 64, 0>(a, nshots, st);
-        case 6: return launch_tile<MODE, 32, 32, 1>(a, nshots, st);
-        case 7: return launch_tile<MODE, 16, 32, 1>(a, nshots, st);
-        case 8: return launch_tile<MODE, 64, 32, 1>(a, nshots, st);
-        case 9: return launch_tile<MODE, 32, 32, 2>(a, nshots, st);
-        case 10: return launch_tile<MODE, 16, 32, 2>(a, nshots, st);
-        case 11: return launch_tile<MODE, 8, 32, 2>(a, nshots, st);
+        case 0: return launch_tile<MODE, 32, 32, 2>(a, nshots, cur, pdl, plan, st);
+        case 1: return launch_tile<MODE, 32, 32, 0>(a, nshots, cur, pdl, plan, st);
+        case 2: return launch_tile<MODE, 16, 64, 0>(a, nshots, cur, pdl, plan, st);
+        case 3: return launch_tile<MODE, 16, 32, 0>(a, nshots, cur, pdl, plan, st);
+        case 4: return launch_tile<MODE, 64, 32, 0>(a, nshots, cur, pdl, plan, st);
+        case 5: return launch_tile<MODE, 8, 64, 0>(a, nshots, cur, pdl, plan, st);
+        case 6: return launch_tile<MODE, 32, 32, 1>(a, nshots, cur, pdl, plan, st);
+        case 7: return launch_tile<MODE, 16, 32, 1>(a, nshots, cur, pdl, plan, st);
+        case 8: return launch_tile<MODE, 64, 32, 1>(a, nshots, cur, pdl, plan, st);
+        case 9: return launch_tile<MODE, 32, 32, 2>(a, nshots, cur, pdl, plan, st);
+        case 10: return launch_tile<MODE, 16, 32, 2>(a, nshots, cur, pdl, plan, st);
+        case 11: return launch_tile<MODE, 8, 32, 2>(a, nshots, cur, pdl, plan, st);
     }
     return set_error(FWI_EINVAL, "unknown tile variant %d", tile);
 }
@@ -821,7 +846,7 @@ static int comp_slot(int mode, int q) {
 }
 
 int launch_step(const fwi_batch *b, int adjoint, int it, bool snap_u_next, int snap_u_slot, bool snap_v,
-                int snap_v_slot, cudaStream_t st) {
+                int snap_v_slot, bool pdl, StepPlan *plan, cudaStream_t st) {
     StepArgs a;
     base_args(b, a);
     a.it = it;
@@ -861,9 +886,9 @@ int launch_step(const fwi_batch *b, int adjoint, int it, bool snap_u_next, int s
     }
     if (adjoint) a.rec_cell = nullptr;  // the adjoint records nothing (solver.py:308-321)
     switch (b->mode) {
-        case FWI_SH: return launch_mode<FWI_SH>(a, b->nshots, b->tile, st);
-        case FWI_PSV: return launch_mode<FWI_PSV>(a, b->nshots, b->tile, st);
-        case FWI_SPIN: return launch_mode<FWI_SPIN>(a, b->nshots, b->tile, st);
+        case FWI_SH: return launch_mode<FWI_SH>(a, b->nshots, b->tile, cur, pdl, plan, st);
+        case FWI_PSV: return launch_mode<FWI_PSV>(a, b->nshots, b->tile, cur, pdl, plan, st);
+        case FWI_SPIN: return launch_mode<FWI_SPIN>(a, b->nshots, b->tile, cur, pdl, plan, st);
     }
     return set_error(FWI_EINVAL, "unknown mode %d", b->mode);
 }
@@ -967,7 +992,7 @@ int multi_prepare(fwi_batch *const *bs, int n, void *ws, int (*check)(const fwi_
 }
 
 template <int MODE, int TX>
-static int launch_multi(const MultiInst *inst, const int *prefix, int nactive, int blocks, int it, int cur,
+static int launch_multi(const MultiInst *inst, const int *prefix, int nactive, int blocks, int it, int cur, bool pdl,
                         cudaStream_t st) {
     using T = Tile<MODE, TX, 32>;
     static bool set = false;
@@ -977,7 +1002,17 @@ static int launch_multi(const MultiInst *inst, const int *prefix, int nactive, i
         if (e != cudaSuccess) return set_error(FWI_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         set = true;
     }
-    step_kernel_multi<MODE, TX><<<blocks, kThreads, T::bytes, st>>>(inst, prefix, nactive, it, cur);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks, 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = T::bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    set_pdl_attr(attr[0], true);
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, step_kernel_multi<MODE, TX>, inst, prefix, nactive, it, cur);
+    if (e != cudaSuccess) return set_error(FWI_ECUDA, "step_kernel_multi launch: %s", cudaGetErrorString(e));
     return check_launch("step_kernel_multi");
 }
 
@@ -998,16 +1033,17 @@ int multi_run(fwi_batch *const *bs, int n, void *ws, int it0, int nsteps, cudaSt
         if (!nactive) break;
         const int cur = (cur0 + (it - it0)) & 1;
         const int blocks = (int)prefix[nactive];
+        const bool pdl = bs[0]->step_overlap != 0 && it > it0;
         if (mode == FWI_SH) {
-            rc = tx == 32 ? launch_multi<FWI_SH, 32>(inst, pdev, nactive, blocks, it, cur, st)
-                 : tx == 16 ? launch_multi<FWI_SH, 16>(inst, pdev, nactive, blocks, it, cur, st)
-                            : launch_multi<FWI_SH, 64>(inst, pdev, nactive, blocks, it, cur, st);
+            rc = tx == 32 ? launch_multi<FWI_SH, 32>(inst, pdev, nactive, blocks, it, cur, pdl, st)
+                 : tx == 16 ? launch_multi<FWI_SH, 16>(inst, pdev, nactive, blocks, it, cur, pdl, st)
+                            : launch_multi<FWI_SH, 64>(inst, pdev, nactive, blocks, it, cur, pdl, st);
         } else if (mode == FWI_PSV) {
-            rc = tx == 32 ? launch_multi<FWI_PSV, 32>(inst, pdev, nactive, blocks, it, cur, st)
-                 : tx == 16 ? launch_multi<FWI_PSV, 16>(inst, pdev, nactive, blocks, it, cur, st)
-                            : launch_multi<FWI_PSV, 64>(inst, pdev, nactive, blocks, it, cur, st);
+            rc = tx == 32 ? launch_multi<FWI_PSV, 32>(inst, pdev, nactive, blocks, it, cur, pdl, st)
+                 : tx == 16 ? launch_multi<FWI_PSV, 16>(inst, pdev, nactive, blocks, it, cur, pdl, st)
+                            : launch_multi<FWI_PSV, 64>(inst, pdev, nactive, blocks, it, cur, pdl, st);
         } else {
-            rc = launch_multi<FWI_SPIN, 32>(inst, pdev, nactive, blocks, it, cur, st);
+            rc = launch_multi<FWI_SPIN, 32>(inst, pdev, nactive, blocks, it, cur, pdl, st);
         }
         for (int i = 0; i < nactive && !rc; i++) bs[order[i]]->cur ^= 1;
     }
@@ -1057,6 +1093,7 @@ int multi_run(fwi_batch *const *bs, int n, void *ws, int it0, int nsteps, cudaSt
 
 struct AdjArgs {
     int nx, nz, pitch, nt, it, nshots;
+    int slot;  // of step it in the segment stores
     FastDiv divnz;
     float cx1, cx2, cz1, cz2, dt, dt2;
     float *sig_out[6];
@@ -1072,7 +1109,7 @@ struct AdjArgs {
 struct AdjMaps {
     CUtensorMap sig[6];  // sig~, stress region box
     CUtensorMap vel[3];  // v~, velocity region box
-    CUtensorMap ef[6];   // forward stress-update terms, interior box
+    CUtensorMap ef[6];   // forward stress-update terms, interior box; the shots of every stored step follow each other
     CUtensorMap lm[4];   // SH: mu | P-SV: lam, mu | spin: lam, mu, nu, mnc; stress region box
     CUtensorMap vp[3];   // dt/rho, sponge (spin: dt/j); velocity region box
 };
@@ -1243,8 +1280,9 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
 #pragma unroll
         for (int q = 0; q < NV; q++) tma_load_3d(sV + q * FV, &m.vel[q], z0 - 4, x0 - 1, shot, &bar[2]);
 #pragma unroll
-        for (int k = 0; k < NE; k++) tma_load_3d(sE + k * TX * TZ, &m.ef[k], z0, x0, shot, &bar[2]);
+        for (int k = 0; k < NE; k++) tma_load_3d(sE + k * TX * TZ, &m.ef[k], z0, x0, (a.slot > 0 ? a.slot * nshots : 0) + shot, &bar[2]);
     };
+    grid_dep_trigger();
     if (tid == 0) {
 #pragma unroll
         for (int b = 0; b < 3; b++) mbar_init(&bar[b], 1);
@@ -1252,15 +1290,18 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
     }
     __syncthreads();
     if (tid == 0) {
+        // the model tile (no step writes it) streams in while the previous step may still be running
         mbar_expect_tx(&bar[0], T::model_bytes);
 #pragma unroll
         for (int f = 0; f < NL; f++) tma_load_2d(sL + f * FS, &m.lm[f], z0 - 4, x0 - 3, &bar[0]);
 #pragma unroll
         for (int p = 0; p < T::NP; p++) tma_load_2d(sP + p * FV, &m.vp[p], z0 - 4, x0 - 1, &bar[0]);
-        if (crank < nshots) {
-            issue_sig(crank);
-            issue_vel(crank);
-        }
+    }
+    // the previous step (adjoint state, gradient sums) is complete from here on
+    grid_dep_wait();
+    if (tid == 0 && crank < nshots) {
+        issue_sig(crank);
+        issue_vel(crank);
     }
 
     float gk[NK][RPW];
@@ -2021,16 +2062,27 @@ static int wide_maps(const fwi_batch *b, WideMaps &m) {
     return rc;
 }
 
+// Tensor maps of a loop of transposed steps, per half of the ping-pong pairs
+// (as StepPlan).
+struct AdjPlan {
+    AdjMaps maps[2];
+    WideMaps wide[2];
+    bool have[2];
+};
+AdjPlan *make_adj_plan() { return new (std::nothrow) AdjPlan(); }
+void free_adj_plan(AdjPlan *p) { delete p; }
+
 // Tensor maps of one transposed step.
 template <int MODE>
-static int adjoint_maps(const fwi_batch *b, const AdjArgs &a, AdjMaps &m) {
+static int adjoint_maps(const fwi_batch *b, long long slot0, int nseg, AdjMaps &m) {
     using T = AdjTile<MODE>;
     using F = Fields<MODE>;
     const int cur = b->cur, nx = b->nx, pitch = b->pitch, ns = b->nshots;
+    const long long field = (long long)ns * nx * pitch;
     int rc = 0;
     for (int f = 0; f < F::NS && !rc; f++) rc = encode_map(&m.sig[f], b->sig[cur][f], 3, pitch, nx, ns, T::SZ, T::SX);
     for (int q = 0; q < F::NV && !rc; q++) rc = encode_map(&m.vel[q], b->vel[cur][q], 3, pitch, nx, ns, T::SZ, T::VX);
-    for (int k = 0; k < T::NE && !rc; k++) rc = encode_map(&m.ef[k], a.ef[k], 3, pitch, nx, ns, T::TZ, T::TX);
+    for (int k = 0; k < T::NE && !rc; k++) rc = encode_map(&m.ef[k], b->seg_e[k] + slot0 * field, 3, pitch, nx, ns * nseg, T::TZ, T::TX);
     const float *lm[4] = {MODE == FWI_SH ? b->mu : b->lam, b->mu, b->nu, b->mnc};
     for (int f = 0; f < T::NL && !rc; f++) rc = encode_map(&m.lm[f], lm[f], 2, pitch, nx, 1, T::SZ, T::SX);
     const float *vp[3] = {b->buo, b->bound, b->buo_j};
@@ -2056,7 +2108,7 @@ static int adjoint_cluster(int nshots, long long tiles, int ctas_per_sm) {
 }
 
 template <int MODE>
-static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, cudaStream_t st) {
+static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPlan *plan, cudaStream_t st) {
     using T = AdjTile<MODE>;
     static bool set = false;
     if (!set) {
@@ -2065,9 +2117,15 @@ static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, cudaStream_t st)
         if (e != cudaSuccess) return set_error(FWI_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         set = true;
     }
-    AdjMaps m;
-    int rc = adjoint_maps<MODE>(b, a, m);
-    if (rc) return rc;
+    AdjMaps &m = plan->maps[b->cur];
+    if (a.slot < 0) {  // more stored shots than a map's coordinate counts: maps of this step's alone
+        const int rc = adjoint_maps<MODE>(b, a.it - b->seg0, 1, m);
+        if (rc) return rc;
+    } else if (!plan->have[b->cur]) {
+        const int rc = adjoint_maps<MODE>(b, 0, b->nseg, m);
+        if (rc) return rc;
+        plan->have[b->cur] = true;
+    }
     const int C = adjoint_cluster(b->nshots, (long long)((b->nz + T::TZ - 1) / T::TZ) * ((b->nx + T::TX - 1) / T::TX),
                                   MODE == FWI_SH ? 4 : MODE == FWI_PSV ? 3 : 2);
     cudaLaunchConfig_t cfg = {};
@@ -2075,19 +2133,20 @@ static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, cudaStream_t st)
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = T::bytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = C;
+    set_pdl_attr(attr[1], true);
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, adjoint_kernel<MODE>, a, m);
     if (e != cudaSuccess) return set_error(FWI_ECUDA, "adjoint_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("adjoint_kernel");
 }
 
-static int launch_adjoint_wide(const fwi_batch *b, const AdjArgs &a, bool pdl, cudaStream_t st) {
+static int launch_adjoint_wide(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPlan *plan, cudaStream_t st) {
     using T = WideTile;
     static bool set = false;
     if (!set) {
@@ -2096,9 +2155,12 @@ static int launch_adjoint_wide(const fwi_batch *b, const AdjArgs &a, bool pdl, c
         if (e != cudaSuccess) return set_error(FWI_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         set = true;
     }
-    WideMaps m;
-    int rc = wide_maps(b, m);
-    if (rc) return rc;
+    WideMaps &m = plan->wide[b->cur];
+    if (!plan->have[b->cur]) {
+        const int rc = wide_maps(b, m);
+        if (rc) return rc;
+        plan->have[b->cur] = true;
+    }
     const int tz = (b->nz + T::TZ - 1) / T::TZ, tx = (b->nx + T::TX - 1) / T::TX;
     const int C = adjoint_cluster(b->nshots, (long long)tz * tx, 2);
     cudaLaunchConfig_t cfg = {};
@@ -2121,7 +2183,7 @@ static int launch_adjoint_wide(const fwi_batch *b, const AdjArgs &a, bool pdl, c
 
 // One transposed step (forward step `it`, adjoint state it+1 -> it) with
 // its gradient terms.
-int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, cudaStream_t st) {
+int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, AdjPlan *plan, cudaStream_t st) {
     AdjArgs a;
     a.nx = b->nx;
     a.nz = b->nz;
@@ -2143,6 +2205,7 @@ int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, cudaStream_t st) {
     for (int q = 0; q < 3; q++) a.vel_out[q] = q < nv ? b->vel[nxt][q] : nullptr;
     const long long field = (long long)b->nshots * b->nx * b->pitch;
     const long long slot = it - b->seg0;
+    a.slot = (long long)b->nshots * b->nseg < (1ll << 31) ? (int)slot : -1;
     for (int k = 0; k < 6; k++) a.ef[k] = k < ne ? b->seg_e[k] + slot * field : nullptr;
     // divergence stores (all components or none: without them the density terms are skipped)
     bool ds = true;
@@ -2170,9 +2233,9 @@ int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, cudaStream_t st) {
     a.g[0] = mode == FWI_SH ? b->stf[1] : b->stf[0];
     a.g[1] = mode == FWI_SH ? nullptr : b->stf[2];
     switch (mode) {
-        case FWI_SH: return launch_adjoint<FWI_SH>(b, a, st);
-        case FWI_PSV: return b->adj_tile == 1 ? launch_adjoint<FWI_PSV>(b, a, st) : launch_adjoint_wide(b, a, pdl, st);
-        default: return launch_adjoint<FWI_SPIN>(b, a, st);
+        case FWI_SH: return launch_adjoint<FWI_SH>(b, a, pdl, plan, st);
+        case FWI_PSV: return b->adj_tile == 1 ? launch_adjoint<FWI_PSV>(b, a, pdl, plan, st) : launch_adjoint_wide(b, a, pdl, plan, st);
+        default: return launch_adjoint<FWI_SPIN>(b, a, pdl, plan, st);
     }
 }
 
