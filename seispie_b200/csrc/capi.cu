@@ -44,6 +44,7 @@ int launch_step(const fwi_batch *b, int adjoint, int it, bool snap_u_next, int s
 int launch_interaction(const fwi_batch *b, int isae, cudaStream_t st);
 int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, AdjPlan *plan, cudaStream_t st);
 int launch_march(const fwi_batch *b, int it, bool pdl, cudaStream_t st);
+int launch_resident(const fwi_batch *b, int it0, int nsteps, cudaStream_t st);
 bool march_supported(const fwi_batch *b);
 int launch_displacement_traces(float *obs, long long ntr, int nt, int it0, int n, double dt, cudaStream_t st);
 int kernel_binary_version(int *v);
@@ -249,9 +250,12 @@ int fwi_run(fwi_batch *b, int adjoint, int it0, int nsteps, void *stream) {
         // every launch after the first follows a row-marching step of this loop
         // directly in the stream, so it may overlap that step's tail
         const bool pdl = b->step_overlap != 0;
-        for (int it = it0; it < it0 + nsteps; it++) {
-            rc = launch_march(b, it, pdl && it > it0, st);
-            if (rc) return rc;
+        rc = launch_resident(b, it0, nsteps, st);  // small grids: all steps in one launch
+        if (rc < 0) return rc;
+        if (rc == 0) b->cur ^= nsteps & 1;
+        for (int it = it0; rc > 0 && it < it0 + nsteps; it++) {
+            const int one = launch_march(b, it, pdl && it > it0, st);
+            if (one) return one;
             b->cur ^= 1;
         }
         const long long ntr = (long long)b->nshots * b->nrec;

@@ -53,6 +53,8 @@
 //     so the per-cell sums are unchanged) and rec_order lists the receivers
 //     by cell.  Each CTA stages the points of its rows in shared-memory
 //     windows and walks them with the march.
+#include <cooperative_groups.h>
+
 #include <atomic>
 #include <cstdio>
 #include <mutex>
@@ -61,6 +63,8 @@
 
 #include "common.cuh"
 #include "stencil.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace fwi {
 
@@ -139,6 +143,16 @@ __device__ __forceinline__ int warp_lower_bound(const int *cell, const int *perm
         const int nlo = k > 0 ? lo + (int)(n * k / 33) + 1 : lo;  // past the last position below
         hi = k < 32 ? lo + (int)(n * (k + 1) / 33) : hi;          // at the first position not below
         lo = nlo;
+    }
+    return lo;
+}
+
+// The same by one thread.
+__device__ __forceinline__ int thread_lower_bound(const int *cell, const int *perm, int lo, int hi, int v) {
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cell[perm ? perm[mid] : mid] < v) lo = mid + 1;
+        else hi = mid;
     }
     return lo;
 }
@@ -688,6 +702,313 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, MODE == FWI_SH ? (WIDE ? 2 :
     }
 }
 
+// ------------------------------------------------- small grids: resident steps
+//
+// All steps of one fwi_run call on a grid whose shots fit the shared memory of
+// a cluster: a cluster of C CTAs holds one shot for the whole call, CTA k the
+// rows [nx k/C, nx (k+1)/C), stress and velocity in shared memory, the model of
+// a thread's cells in its registers.  A thread owns four adjacent columns of up
+// to kResRows consecutive rows, so the x taps of the stencils are read once per
+// row.  Per step: velocity of the own rows and of the three halo rows the D+x
+// taps reach (computed twice, so that only stress is exchanged), a block
+// barrier, stress of the own rows, whose first and last three the owner also
+// writes into the neighbours' halo rows (distributed shared memory, two copies
+// by the parity of the step), a cluster barrier.  Sources and receivers as in
+// march_kernel: the points of a thread's cells are ranges of the cell-sorted
+// lists, found once per call.  The arithmetic per cell is march_kernel's.
+//
+// A launched step cannot be shorter than a launch and a pass through L2, 5.6 us
+// (SH) to 8 us (P-SV) here; a resident one costs its arithmetic, bound by the
+// latency of 16 warps' shared-memory loads and packed operations, and two
+// barriers: one SH shot on 256 x 256 5.9 -> 2.8 us, P-SV 183 x 270, 3 shots
+// 8.5 -> 4.8 us, 256 x 128, 16 shots 12.4 -> 5.8 us, 64 x 64, 64 shots 13.4 ->
+// 3.4 us a step.
+
+constexpr int kResThreads = 512;
+constexpr int kResPts = 64;  // source values and receiver numbers staged in shared memory
+
+struct ResidentArgs {
+    int nx, nz, pitch, nt, it0, nsteps, nrec;
+    int rows_max;           // rows of a CTA, at most
+    int groups, segs;       // column groups of four per row; row segments (threads = groups x segs)
+    float cx1, cx2, cz1, cz2, dt;
+    const float *sig_in[3];
+    float *sig_out[3];
+    const float *vel_in[2];
+    float *vel_out[2];
+    const float *buo, *bound;
+    const float *ip[2];
+    const int *inj_ptr, *inj_cell, *inj_row;
+    const float *stf[2];
+    const int *rec_cell, *rec_order;
+    float *obs[2];
+};
+
+// Floats of shared memory: stress rows (own, and two copies of the three halo
+// rows on either side) and velocity rows of RL floats, then the staged points.
+template <int MODE>
+static size_t resident_bytes(int rows, int pitch) {
+    using F = Fields<MODE>;
+    return sizeof(float) * ((size_t)(F::NS * (rows + 12) + F::NV * (rows + 3)) * (pitch + 8) +
+                            (size_t)kResPts * (2 * F::NINJ + 3));
+}
+
+template <int MODE, int I>
+__global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_constant__ ResidentArgs a) {
+    using F = Fields<MODE>;
+    constexpr int NS = F::NS, NV = F::NV, NINJ = F::NINJ;
+    constexpr int FX0 = 0, FX1 = MODE == FWI_SH ? 0 : 2, FZ = 1;
+    extern __shared__ __align__(128) float smem[];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int nx = a.nx, nz = a.nz, pitch = a.pitch, nt = a.nt, RL = pitch + 8, RM = a.rows_max;
+    const int shot = blockIdx.y, tid = threadIdx.x;
+    const int row0 = (int)((long long)nx * rank / C), n = (int)((long long)nx * (rank + 1) / C) - row0;
+    const int FS = (RM + 12) * RL, FV = (RM + 3) * RL;  // field strides
+    // stress row q = 0 .. n+5 is grid row row0-3+q; the halo rows q < 3 and q >= n+3 of an odd step sit in the
+    // last six rows of the field.  Velocity row q = 0 .. n+2 is grid row row0-1+q.
+    float *const S = smem, *const V = smem + NS * FS;
+    float *const pts = V + NV * FV;  // source values [2][NINJ][kResPts]; source cells, receiver numbers and cells
+    int *const i_cell = reinterpret_cast<int *>(pts + 2 * NINJ * kResPts), *const r_id = i_cell + kResPts,
+              *const r_cell = r_id + kResPts;
+    const int cg4 = tid % a.groups, seg = tid / a.groups, j0 = 4 * cg4;
+    const bool work = seg < a.segs;
+    const Coef kx{bc2(a.cx1), bc2(-a.cx2)}, kz{bc2(a.cz1), bc2(-a.cz2)};
+    const Q4 dt4{bc2(a.dt), bc2(a.dt)};
+    const long long soff = (long long)shot * nx * pitch;
+    bool zm[4], zp[4], zin[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const int c = j0 + e;
+        zm[e] = c >= 2 && c < nz - 2;
+        zp[e] = c >= 1 && c < nz - 2;
+        zin[e] = c < nz;
+    }
+    // this thread's velocity rows [v0, v0+nv) of n+3 and stress rows [s0, s0+ns) of n, as local rows
+    const int iv = (n + 3 + a.segs - 1) / a.segs, is = (n + a.segs - 1) / a.segs;
+    const int v0 = seg * iv, nv = work ? min(iv, n + 3 - v0) : 0;
+    const int s0 = seg * is, ns = work ? min(is, n - s0) : 0;
+
+    // ---- state into shared memory (zero outside the grid)
+    for (int q = tid; q < (n + 6) * a.groups; q += kResThreads) {
+        const int r = q / a.groups, c = 4 * (q - r * a.groups), gr = row0 - 3 + r;
+        const bool in = gr >= 0 && gr < nx;
+#pragma unroll
+        for (int f = 0; f < NS; f++) {
+            const Q4 v = in ? ld4(a.sig_in[f] + soff + (long long)gr * pitch + c) : zero4();
+            st4(S + f * FS + r * RL + 4 + c, v);
+            // the odd copies of halo rows outside the grid stay zero; the others are written by the first step
+            if (r < 3) st4(S + f * FS + (RM + 6 + r) * RL + 4 + c, zero4());
+            if (r >= n + 3) st4(S + f * FS + (RM + 9 + r - n - 3) * RL + 4 + c, zero4());
+        }
+        if (r >= 2 && r < n + 5) {
+#pragma unroll
+            for (int c2 = 0; c2 < NV; c2++)
+                st4(V + c2 * FV + (r - 2) * RL + 4 + c, in ? ld4(a.vel_in[c2] + soff + (long long)gr * pitch + c) : zero4());
+        }
+    }
+    // ---- model of this thread's cells (zero in the padding columns, which keeps them zero)
+    Q4 buo[I], bnd[I], ip0[I], ip1[I];
+    // points of its velocity cells: first entry and count of the two lists
+    int inj_lo[I], rec_lo[I];
+    unsigned cnt[I];  // injection count | receiver count << 16
+    const bool rec_on = a.rec_order && a.nrec > 0 && (a.obs[0] || (NV > 1 && a.obs[1]));
+    int p0 = 0, p1 = 0;
+    if (a.inj_ptr) {
+        p0 = a.inj_ptr[shot];
+        p1 = a.inj_ptr[shot + 1];
+    }
+    // the entries of the CTA's rows, of which the first kResPts are staged
+    const int clo = max(row0 - 1, 0) * nz, chi = min(row0 + n + 2, nx) * nz;
+    const int il = thread_lower_bound(a.inj_cell, nullptr, p0, p1, clo), ih = thread_lower_bound(a.inj_cell, nullptr, il, p1, chi);
+    const int rl = rec_on ? thread_lower_bound(a.rec_cell, a.rec_order, 0, a.nrec, row0 * nz) : 0;
+    const int rh = rec_on ? thread_lower_bound(a.rec_cell, a.rec_order, rl, a.nrec, (row0 + n) * nz) : 0;
+    const int ni = min(ih - il, kResPts), nr = min(rh - rl, kResPts);
+#pragma unroll
+    for (int k = 0; k < I; k++) {
+        const int gr = row0 - 1 + v0 + k;
+        const bool in = k < nv && gr >= 0 && gr < nx;
+        buo[k] = in ? keep4(ldg4(a.buo + (long long)gr * pitch + j0), zin) : zero4();
+        bnd[k] = in ? keep4(ldg4(a.bound + (long long)gr * pitch + j0), zin) : zero4();
+        const int gs = row0 + s0 + k;
+        ip0[k] = k < ns ? keep4(ldg4(a.ip[0] + (long long)gs * pitch + j0), zin) : zero4();
+        if (MODE == FWI_PSV) ip1[k] = k < ns ? keep4(ldg4(a.ip[1] + (long long)gs * pitch + j0), zin) : zero4();
+        inj_lo[k] = rec_lo[k] = 0;
+        cnt[k] = 0;
+        if (in && j0 < nz) {
+            const int c0 = gr * nz + j0, c1 = gr * nz + min(j0 + 4, nz);
+            inj_lo[k] = thread_lower_bound(a.inj_cell, nullptr, il, ih, c0);
+            cnt[k] = thread_lower_bound(a.inj_cell, nullptr, inj_lo[k], ih, c1) > inj_lo[k] ? 1u : 0u;
+            if (gr >= row0 && gr < row0 + n && rh > rl) {
+                rec_lo[k] = thread_lower_bound(a.rec_cell, a.rec_order, rl, rh, c0);
+                cnt[k] |= thread_lower_bound(a.rec_cell, a.rec_order, rec_lo[k], rh, c1) > rec_lo[k] ? 2u : 0u;
+            }
+        }
+    }
+    // source values of a step, staged one step ahead
+    auto stage = [&](int it) {
+        if (tid < ni) {
+            const long long src = (long long)a.inj_row[il + tid] * nt + it;
+#pragma unroll
+            for (int q = 0; q < NINJ; q++) pts[((it & 1) * NINJ + q) * kResPts + tid] = a.stf[q][src];
+        }
+    };
+    stage(a.it0);
+    if (tid < ni) i_cell[tid] = a.inj_cell[il + tid];
+    if (tid < nr) {
+        r_id[tid] = a.rec_order[rl + tid];
+        r_cell[tid] = a.rec_cell[r_id[tid]];
+    }
+    cluster.sync();
+
+    float *const up = rank > 0 ? cluster.map_shared_rank(S, rank - 1) : nullptr;
+    float *const down = rank + 1 < C ? cluster.map_shared_rank(S, rank + 1) : nullptr;
+    const int n_up = row0 - (rank > 0 ? (int)((long long)nx * (rank - 1) / C) : 0);  // rows of the CTA above
+    for (int step = 0; step < a.nsteps; step++) {
+        const int it = a.it0 + step, par = step & 1;
+        // stress row q of this step at this thread's columns
+        auto srow = [&](int q) -> float * {
+            int r = q;
+            if (par && q < 3) r = RM + 6 + q;
+            if (par && q >= n + 3) r = RM + 9 + q - n - 3;
+            return S + r * RL + 4 + j0;
+        };
+        // ---- velocity
+        if (nv > 0) {
+            Q4 w0[4], w1[4];  // D-x windows
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const float *s = srow(v0 + k);
+                w0[k] = ld4(s + FX0 * FS);
+                if (NV > 1) w1[k] = ld4(s + FX1 * FS);
+            }
+#pragma unroll
+            for (int k = 0; k < I; k++) {
+                if (k < nv) {
+                    const int gr = row0 - 1 + v0 + k;
+                    const float *s = srow(v0 + k + 3), *sc = srow(v0 + k + 2);
+                    w0[(k + 3) & 3] = ld4(s + FX0 * FS);
+                    if (NV > 1) w1[(k + 3) & 3] = ld4(s + FX1 * FS);
+                    if (gr >= 0 && gr < nx) {
+                        const Q4 cz = ld4(sc + FZ * FS);
+                        Q4 ds[NV], vn[NV];
+                        if constexpr (MODE == FWI_SH) {
+                            ds[0] = keep4(dzm4(kz, sc + FZ * FS, cz), zm);
+                        } else {
+                            ds[0] = keep4(dzm4(kz, sc + FX1 * FS, w1[(k + 2) & 3]), zm);
+                            ds[NV - 1] = keep4(dzm4(kz, sc + FZ * FS, cz), zm);
+                        }
+                        if (gr >= 2 && gr < nx - 2) {
+                            ds[0] = add4(fdx(kx, w0[(k + 2) & 3], w0[(k + 1) & 3], w0[(k + 3) & 3], w0[k & 3]), ds[0]);
+                            if (NV > 1)
+                                ds[NV - 1] = add4(fdx(kx, w1[(k + 2) & 3], w1[(k + 1) & 3], w1[(k + 3) & 3], w1[k & 3]),
+                                                  ds[NV - 1]);
+                        }
+                        if (cnt[k] & 1) {  // sources, summed per cell in entry order (stf_dsy / stf_dsxz, solver.py:78-93)
+                            Q4 acc[NINJ];
+#pragma unroll
+                            for (int q = 0; q < NINJ; q++) acc[q] = zero4();
+                            const int base = gr * nz + j0, end = gr * nz + min(j0 + 4, nz);
+                            for (int e = inj_lo[k]; e < ih; e++) {
+                                const int at = e - il, cell = at < kResPts ? i_cell[at] : a.inj_cell[e];
+                                if (cell >= end) break;
+#pragma unroll
+                                for (int q = 0; q < NINJ; q++) {
+                                    const float val = at < kResPts ? pts[((it & 1) * NINJ + q) * kResPts + at]
+                                                                   : a.stf[q][(long long)a.inj_row[e] * nt + it];
+#pragma unroll
+                                    for (int x = 0; x < 4; x++)
+                                        if (cell - base == x) elem(acc[q], x) += val;
+                                }
+                            }
+#pragma unroll
+                            for (int q = 0; q < NV; q++) ds[q] = add4(ds[q], acc[q]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < NV; c++) {
+                            float *v = V + c * FV + (v0 + k) * RL + 4 + j0;
+                            vn[c] = mul4(bnd[k], fma4(ds[c], buo[k], ld4(v)));
+                            st4(v, vn[c]);
+                        }
+                        if (cnt[k] & 2) {  // receivers record the new velocity (save_obs, solver.py:151-156)
+                            const int base = gr * nz + j0, end = gr * nz + min(j0 + 4, nz);
+                            for (int e = rec_lo[k]; e < rh; e++) {
+                                const int at = e - rl, id = at < kResPts ? r_id[at] : a.rec_order[e];
+                                const int cell = at < kResPts ? r_cell[at] : a.rec_cell[id];
+                                if (cell >= end) break;
+                                const long long o = ((long long)shot * a.nrec + id) * nt + it;
+#pragma unroll
+                                for (int x = 0; x < 4; x++)
+                                    if (cell - base == x) {
+#pragma unroll
+                                        for (int q = 0; q < NV; q++)
+                                            if (a.obs[q]) a.obs[q][o] = elem(vn[q], x);
+                                    }
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (step + 1 < a.nsteps) stage(it + 1);
+        // ---- stress
+        if (ns > 0) {
+            Q4 w[NV][4];  // velocity rows s-1 .. s+2
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+#pragma unroll
+                for (int c = 0; c < NV; c++) w[c][k] = ld4(V + c * FV + (s0 + k) * RL + 4 + j0);
+#pragma unroll
+            for (int k = 0; k < I; k++) {
+                if (k < ns) {
+                    const int gs = row0 + s0 + k;
+                    Q4 ex[NV], ez[NV];
+#pragma unroll
+                    for (int c = 0; c < NV; c++) {
+                        const float *v = V + c * FV + (s0 + k) * RL + 4 + j0;
+                        w[c][(k + 3) & 3] = ld4(v + 3 * RL);
+                        ez[c] = keep4(dzp4(kz, v + RL, w[c][(k + 1) & 3]), zp);
+                        if (gs >= 1 && gs < nx - 2) ex[c] = fdx(kx, w[c][(k + 2) & 3], w[c][(k + 1) & 3], w[c][(k + 3) & 3], w[c][k & 3]);
+                        else ex[c] = zero4();
+                    }
+                    float *s = S + (s0 + k + 3) * RL + 4 + j0;
+                    Q4 o[NS];
+                    if constexpr (MODE == FWI_SH) {
+                        const Q4 dm = mul4(dt4, ip0[k]);
+                        o[0] = fma4(dm, ex[0], ld4(s));
+                        o[1] = fma4(dm, ez[0], ld4(s + FS));
+                    } else {
+                        const Q4 two{bc2(2.f), bc2(2.f)};
+                        const Q4 l2m = fma4(two, ip1[k], ip0[k]);
+                        o[0] = fma4(dt4, fma4(l2m, ex[0], mul4(ip0[k], ez[NV - 1])), ld4(s));
+                        o[1] = fma4(dt4, fma4(ip0[k], ex[0], mul4(l2m, ez[NV - 1])), ld4(s + FS));
+                        o[NS - 1] = fma4(dt4, mul4(ip1[k], add4(ez[0], ex[NV - 1])), ld4(s + (NS - 1) * FS));
+                    }
+                    const int q = s0 + k;
+#pragma unroll
+                    for (int f = 0; f < NS; f++) {
+                        st4(s + f * FS, o[f]);
+                        // the neighbours' halo rows of the next step (even steps read the rows in place)
+                        if (up && q < 3) st4(up + f * FS + ((par ? n_up + 3 : RM + 9) + q) * RL + 4 + j0, o[f]);
+                        if (down && q >= n - 3) st4(down + f * FS + ((par ? 0 : RM + 6) + q - n + 3) * RL + 4 + j0, o[f]);
+                    }
+                }
+            }
+        }
+        cluster.sync();
+    }
+    // ---- state back
+    for (int q = tid; q < n * a.groups; q += kResThreads) {
+        const int r = q / a.groups, c = 4 * (q - r * a.groups);
+        const long long g = soff + (long long)(row0 + r) * pitch + c;
+#pragma unroll
+        for (int f = 0; f < NS; f++) st4(a.sig_out[f] + g, ld4(S + f * FS + (r + 3) * RL + 4 + c));
+#pragma unroll
+        for (int c2 = 0; c2 < NV; c2++) st4(a.vel_out[c2] + g, ld4(V + c2 * FV + (r + 1) * RL + 4 + c));
+    }
+}
+
 // Displacement traces from velocity traces: u(it) = u(it-1) + v(it) dt over
 // steps [it0, it0+n) of every trace ([trace][nt]), u(it0-1) being the
 // trace's value before it0 (0 at it0 = 0) -- the displacement update of
@@ -808,6 +1129,194 @@ static int launch_march_any(MarchArgs &a, int nthr, int want, int cap, bool pdl,
                    : launch_march_mode<MODE, 1, false>(a, nthr, want, cap, pdl, st);
     return seg ? launch_march_mode<MODE, 0, true>(a, nthr, want, cap, pdl, st)
                : launch_march_mode<MODE, 0, false>(a, nthr, want, cap, pdl, st);
+}
+
+// ------------------------------------------------------------ resident steps
+
+constexpr int kResMinSteps = 24;  // fewer steps in one call are launched one by one
+
+// Clusters of csize CTAs of the resident kernel the GPU holds at once (0: none).
+template <int MODE, int I>
+static int resident_clusters(int csize, size_t bytes) {
+    static std::mutex lock;
+    struct Known {
+        int csize, clusters;
+        size_t bytes;
+    };
+    static std::vector<Known> known;
+    std::lock_guard<std::mutex> hold(lock);
+    const auto kernel = resident_kernel<MODE, I>;
+    if (known.empty() &&
+        (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+        cudaGetLastError();
+        return 0;
+    }
+    for (const Known &k : known)
+        if (k.csize == csize && k.bytes == bytes) return k.clusters;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(csize, 1, 1);
+    cfg.blockDim = dim3(kResThreads, 1, 1);
+    cfg.dynamicSmemBytes = bytes;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();  // a cluster this large or this much shared memory: not available
+        n = 0;
+    }
+    if (known.size() >= 1024) known.clear();
+    known.push_back(Known{csize, n, bytes});
+    return n;
+}
+
+template <int MODE, int I>
+static int launch_resident_kernel(const ResidentArgs &a, int csize, int nshots, size_t bytes, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(csize, nshots, 1);
+    cfg.blockDim = dim3(kResThreads, 1, 1);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, resident_kernel<MODE, I>, a);
+    if (e != cudaSuccess) return set_error(FWI_ECUDA, "resident_kernel launch: %s", cudaGetErrorString(e));
+    return check_launch("resident_kernel");
+}
+
+template <int MODE>
+static int resident_clusters_i(int i, int csize, size_t bytes) {
+    switch (i) {
+        case 1: return resident_clusters<MODE, 1>(csize, bytes);
+        case 2: return resident_clusters<MODE, 2>(csize, bytes);
+        case 3: return resident_clusters<MODE, 3>(csize, bytes);
+        default: return resident_clusters<MODE, 4>(csize, bytes);
+    }
+}
+
+// Microseconds of a step, fitted to measurements and indexed by wave type (SH,
+// P-SV).  Launched: a + b per cell of the batch (one SH shot on 256 x 256 5.9,
+// 16 shots 10.6; P-SV 183 x 270, 3 shots 8.5, 256 x 128, 16 shots 12.4).
+// Resident: a + b per velocity and per stress row of a thread (SH 256 x 256 on
+// 16 CTAs, 3 + 2 rows, 2.8; on 9 CTAs, 4 + 4 rows, 4.0; P-SV 128 x 96 on 16
+// CTAs, 1 + 1 rows, 2.4; 64 x 64 on 2 CTAs, 2 + 2 rows, 3.4; 183 x 270 on 16
+// CTAs, 3 + 2 rows, 4.8), more where the model of 3 or 4 rows of P-SV cells
+// spills registers (256 x 128 on 6 CTAs, 3 + 3 rows, 5.8; 183 x 270 on 8 CTAs,
+// 4 + 4 rows, 8.2), times the waves of clusters that the GPU does not hold at
+// once.  Resident wins for every batch that one wave holds and loses to
+// launched steps from three or four waves on.
+static double launched_us(int mode, double cells) {
+    return mode == FWI_SH ? 5.5 + 4.9e-6 * cells : 7.5 + 8.3e-6 * cells;
+}
+static double resident_us(int mode, int vel_rows, int stress_rows) {
+    if (mode == FWI_SH) return 0.75 + 0.4 * (vel_rows + stress_rows);
+    const double spill = vel_rows == 4 ? 2.0 : vel_rows == 3 && stress_rows == 3 ? 0.9 : 0.0;
+    return 1.0 + 0.65 * (vel_rows + stress_rows) + spill;
+}
+
+// The cluster size and rows per thread that finish a call first, or false
+// where launched steps do or a shot does not fit.
+struct ResidentPlan {
+    int csize, rows, groups, segs, i;
+    size_t bytes;
+};
+template <int MODE>
+static bool resident_plan(const fwi_batch *b, ResidentPlan *out) {
+    const int groups = b->pitch / 4;
+    if (groups > kResThreads) return false;
+    double best = 0.9 * launched_us(MODE, (double)b->nx * b->pitch * b->nshots);
+    bool found = false;
+    for (int c = 1; c <= 16; c++) {
+        const int rows = (b->nx + c - 1) / c;
+        if (b->nx / c < 3) break;  // the three rows a neighbour needs come from one CTA
+        const int segs = kResThreads / groups, i = (rows + 3 + segs - 1) / segs, is = (rows + segs - 1) / segs;
+        const size_t bytes = resident_bytes<MODE>(rows, b->pitch);
+        if (i > 4 || bytes > kMaxSmem) continue;
+        const int n = resident_clusters_i<MODE>(i, c, bytes);
+        if (n < 1) continue;
+        const double t = (b->nshots + n - 1) / n * resident_us(MODE, i, is);
+        if (t < best) {
+            best = t;
+            found = true;
+            *out = ResidentPlan{c, rows, groups, segs, i, bytes};
+        }
+    }
+    return found;
+}
+
+// All steps [it0, it0 + nsteps) of a displacement-free forward batch on the
+// resident kernel, the state going from half cur to the half that many
+// single steps would end in; 1 if the batch is left to launched steps.
+int launch_resident(const fwi_batch *b, int it0, int nsteps, cudaStream_t st) {
+    const int mode = b->mode;
+    // segment stores come from launched steps
+    const bool seg = it0 + nsteps > b->seg0 && it0 < b->seg0 + b->nseg;
+    if (nsteps < kResMinSteps || seg || b->ring || b->ctas_per_sm) return 1;
+    ResidentPlan p;
+    if (!(mode == FWI_SH ? resident_plan<FWI_SH>(b, &p) : resident_plan<FWI_PSV>(b, &p))) return 1;
+    ResidentArgs a;
+    a.nx = b->nx;
+    a.nz = b->nz;
+    a.pitch = b->pitch;
+    a.nt = b->nt;
+    a.it0 = it0;
+    a.nsteps = nsteps;
+    a.nrec = b->nrec;
+    a.rows_max = p.rows;
+    a.groups = p.groups;
+    a.segs = p.segs;
+    a.cx1 = (float)(9.0 / (8.0 * (double)b->dx));
+    a.cx2 = (float)(1.0 / (24.0 * (double)b->dx));
+    a.cz1 = (float)(9.0 / (8.0 * (double)b->dz));
+    a.cz2 = (float)(1.0 / (24.0 * (double)b->dz));
+    a.dt = (float)b->dt;
+    const int cur = b->cur, end = cur ^ (nsteps & 1), ns = mode == FWI_SH ? 2 : 3, nv = mode == FWI_SH ? 1 : 2;
+    for (int f = 0; f < 3; f++) {
+        a.sig_in[f] = f < ns ? b->sig[cur][f] : nullptr;
+        a.sig_out[f] = f < ns ? b->sig[end][f] : nullptr;
+    }
+    for (int q = 0; q < 2; q++) {
+        const bool on = q < nv;
+        a.vel_in[q] = on ? b->vel[cur][q] : nullptr;
+        a.vel_out[q] = on ? b->vel[end][q] : nullptr;
+        a.obs[q] = on ? b->obs[comp_slot_of(mode, q)] : nullptr;
+    }
+    a.buo = b->buo;
+    a.bound = b->bound;
+    a.ip[0] = mode == FWI_SH ? b->mu : b->lam;
+    a.ip[1] = mode == FWI_SH ? nullptr : b->mu;
+    a.inj_ptr = b->inj_ptr;
+    a.inj_cell = b->inj_cell;
+    a.inj_row = b->inj_row;
+    a.stf[0] = mode == FWI_SH ? b->stf[1] : b->stf[0];
+    a.stf[1] = mode == FWI_SH ? nullptr : b->stf[2];
+    a.rec_cell = b->rec_cell;
+    a.rec_order = b->rec_order;
+    const int n = b->nshots;
+    if (mode == FWI_SH) {
+        switch (p.i) {
+            case 1: return launch_resident_kernel<FWI_SH, 1>(a, p.csize, n, p.bytes, st);
+            case 2: return launch_resident_kernel<FWI_SH, 2>(a, p.csize, n, p.bytes, st);
+            case 3: return launch_resident_kernel<FWI_SH, 3>(a, p.csize, n, p.bytes, st);
+            default: return launch_resident_kernel<FWI_SH, 4>(a, p.csize, n, p.bytes, st);
+        }
+    }
+    switch (p.i) {
+        case 1: return launch_resident_kernel<FWI_PSV, 1>(a, p.csize, n, p.bytes, st);
+        case 2: return launch_resident_kernel<FWI_PSV, 2>(a, p.csize, n, p.bytes, st);
+        case 3: return launch_resident_kernel<FWI_PSV, 3>(a, p.csize, n, p.bytes, st);
+        default: return launch_resident_kernel<FWI_PSV, 4>(a, p.csize, n, p.bytes, st);
+    }
 }
 
 int launch_march(const fwi_batch *b, int it, bool pdl, cudaStream_t st) {
