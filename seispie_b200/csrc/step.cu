@@ -1147,7 +1147,7 @@ struct AdjTile {
 // order.  adj_collect compacts up to kThreads entries [base, p1) into the
 // list (block-wide; the count it returns is block-uniform) and may run
 // while the staging copies are in flight; adj_apply adds them once v~ has
-// landed and the list is visible to thread 0.
+// landed and the list is visible to the first warp.
 // adj_fetch: this thread's entry base + tid (its shared-memory location in
 // the staged v~, or -1, and its u~ values); no barrier, so it can be issued
 // well before adj_compact needs it.
@@ -1202,13 +1202,32 @@ __device__ __forceinline__ int adj_collect(const AdjArgs &a, int base, int p1, i
     return adj_compact<MODE>(loc, val, sLoc, sVal, sWarp);
 }
 
-template <int MODE>
+// Add the n listed entries to the staged v~ (first warp).  32 entries in
+// strictly increasing locations, the usual case, are distinct cells and go in
+// one pass; any other 32 are summed one by one in entry order, since they may
+// share a cell.  (One thread adding every entry made the tiles with receivers
+// the last to finish: P-SV 512 x 512, 32 shots 125 -> 116 us a step, 256 x
+// 128, 16 shots 19.6 -> 18.1 us.)
+template <int NINJ, int FV>
 __device__ __forceinline__ void adj_apply(float *sV, int n, const int *sLoc, const float *sVal, float dt) {
-    if (threadIdx.x != 0) return;
-    for (int q = 0; q < n; q++) {
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    for (int base = 0; base < n; base += 32) {
+        const int q = base + lane;
+        const int loc = q < n ? sLoc[q] : 0x7fffffff - 32 + lane;
+        const int prev = __shfl_up_sync(0xffffffffu, loc, 1);
+        if (__all_sync(0xffffffffu, lane == 0 || loc > prev)) {
+            if (q < n) {
 #pragma unroll
-        for (int c = 0; c < Fields<MODE>::NINJ; c++)
-            sV[c * AdjTile<MODE>::FV + sLoc[q]] += dt * sVal[c * kThreads + q];
+                for (int c = 0; c < NINJ; c++) sV[c * FV + loc] += dt * sVal[c * kThreads + q];
+            }
+        } else if (lane == 0) {
+            for (int r = base; r < min(base + 32, n); r++) {
+#pragma unroll
+                for (int c = 0; c < NINJ; c++) sV[c * FV + sLoc[r]] += dt * sVal[c * kThreads + r];
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -1395,9 +1414,9 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
                 }
             }
         }
-        // v~ and the forward strain of this shot; u~ enters v~ (thread 0)
+        // v~ and the forward strain of this shot; u~ enters v~ (first warp)
         ok = mbar_wait(&bar[2], i & 1);
-        if (single && ok) adj_apply<MODE>(sV, n_in, sLoc, sVal, dt);
+        if (single && ok) adj_apply<F::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicExch(&g_device_status, 1);
             mbar_wait(&bar[2], i & 1);
@@ -1408,7 +1427,7 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
                 __syncthreads();
                 const int n = adj_collect<MODE>(a, base, p1, x0, z0, sLoc, sVal, sWarp);
                 __syncthreads();
-                adj_apply<MODE>(sV, n, sLoc, sVal, dt);
+                adj_apply<F::NINJ, FV>(sV, n, sLoc, sVal, dt);
             }
             __syncthreads();
         }
@@ -1662,14 +1681,6 @@ __device__ __forceinline__ void wide_fetch(const AdjArgs &a, int base, int p1, i
     }
 }
 
-__device__ __forceinline__ void wide_apply(float *sV, int n, const int *sLoc, const float *sVal, float dt) {
-    if (threadIdx.x != 0) return;
-    for (int q = 0; q < n; q++) {
-        sV[sLoc[q]] += dt * sVal[q];
-        sV[WideTile::FV + sLoc[q]] += dt * sVal[kThreads + q];
-    }
-}
-
 __device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 __device__ __forceinline__ void st2(float *p, float x, float y) { *reinterpret_cast<float2 *>(p) = make_float2(x, y); }
 
@@ -1810,9 +1821,9 @@ __global__ void __launch_bounds__(kThreads, 2)
             s4[F4] = zz;
             s4[2 * F4] = xz;
         }
-        // v~ of this shot; u~ enters v~ (thread 0)
+        // v~ of this shot; u~ enters v~ (first warp)
         ok = mbar_wait(&bar[2], i & 1);
-        if (single && ok) wide_apply(sV, n_in, sLoc, sVal, dt);
+        if (single && ok) adj_apply<T::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicExch(&g_device_status, 1);
             mbar_wait(&bar[2], i & 1);
@@ -1826,7 +1837,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 wide_fetch(a, base, p1, x0, z0, loc, val);
                 const int n = adj_compact<FWI_PSV>(loc, val, sLoc, sVal, sWarp);
                 __syncthreads();
-                wide_apply(sV, n, sLoc, sVal, dt);
+                adj_apply<T::NINJ, FV>(sV, n, sLoc, sVal, dt);
             }
             __syncthreads();
         }
