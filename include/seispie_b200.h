@@ -125,9 +125,9 @@ typedef struct fwi_batch {
      * as many as fit).  A smaller grid leaves room on every SM for another
      * kernel running concurrently on a second stream. */
     int ctas_per_sm;
-    /* P-SV transposed step (fwi_run_transposed): 0 = tiles of 32 x 64 cells,
-     * two z columns per thread; 1 = tiles of 32 x 32 cells, one column per
-     * thread.  Same adjoint fields bit for bit. */
+    /* P-SV transposed step (fwi_run_transposed): 0 = tiles chosen by the size
+     * of the batch (32 x 64 cells with two z columns per thread, or 32, 16 or
+     * 8 rows of 32 with one); 1 = 32 x 32.  Same adjoint fields bit for bit. */
     int adj_tile;
     /* 1: programmatic dependent launch between the steps of one fwi_run,
      * fwi_run_transposed or fwi_multi_run call (all but the tile variants

@@ -208,7 +208,7 @@ class ExactAdjoint:
             self.seg_ds[c] = torch.empty((self.K2,) + shape, dtype=torch.float32, device=dev)
         self.overlap = bool(overlap) and self.nseg > 1
         self.overlap_ctas = int(overlap_ctas)
-        self.adj_tile = 0  # P-SV transposed step: 0 = 32 x 64 tiles, 1 = 32 x 32 tiles (same values)
+        self.adj_tile = 0  # P-SV transposed step: 0 = tiles by size, 1 = 32 x 32 tiles (same values)
         if self.overlap:
             self.seg_e2 = [None if t is None else torch.empty_like(t) for t in self.seg_e]
             self.seg_ds2 = [None if t is None else torch.empty_like(t) for t in self.seg_ds]

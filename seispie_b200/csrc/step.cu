@@ -37,6 +37,8 @@
 // outside the grid or in row padding ever reaches a result.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include <type_traits>
 
 #include <cstdio>
@@ -1114,11 +1116,11 @@ struct AdjMaps {
     CUtensorMap vp[3];   // dt/rho, sponge (spin: dt/j); velocity region box
 };
 
-template <int MODE>
+template <int MODE, int ROWS>
 struct AdjTile {
     using F = Fields<MODE>;
-    // spin holds twice the fields: 16 x 32 tiles keep two CTAs per SM
-    static constexpr int TX = MODE == FWI_SPIN ? 16 : 32, TZ = 32;
+    // ROWS: 8, 16 or 32 (spin holds twice the fields: up to 16 rows keep two CTAs per SM)
+    static constexpr int TX = ROWS, TZ = 32;
     static constexpr int SX = TX + 6, SZ = TZ + 8, VX = TX + 3, RVZ = TZ + 3;
     static constexpr int FS = (SX * SZ + 31) / 32 * 32, FV = (VX * SZ + 31) / 32 * 32;
     static constexpr int NL = MODE == FWI_SH ? 1 : MODE == FWI_PSV ? 2 : 4;  // stiffness fields
@@ -1151,10 +1153,10 @@ struct AdjTile {
 // adj_fetch: this thread's entry base + tid (its shared-memory location in
 // the staged v~, or -1, and its u~ values); no barrier, so it can be issued
 // well before adj_compact needs it.
-template <int MODE>
+template <int MODE, int ROWS>
 __device__ __forceinline__ void adj_fetch(const AdjArgs &a, int base, int p1, int x0, int z0, int &loc,
                                           float (&val)[Fields<MODE>::NINJ]) {
-    using T = AdjTile<MODE>;
+    using T = AdjTile<MODE, ROWS>;
     const int e = base + (int)threadIdx.x;
     loc = -1;
 #pragma unroll
@@ -1193,12 +1195,12 @@ __device__ __forceinline__ int adj_compact(int loc, const float (&val)[Fields<MO
     return n;
 }
 
-template <int MODE>
+template <int MODE, int ROWS>
 __device__ __forceinline__ int adj_collect(const AdjArgs &a, int base, int p1, int x0, int z0, int *sLoc,
                                            float *sVal, int *sWarp) {
     int loc;
     float val[Fields<MODE>::NINJ];
-    adj_fetch<MODE>(a, base, p1, x0, z0, loc, val);
+    adj_fetch<MODE, ROWS>(a, base, p1, x0, z0, loc, val);
     return adj_compact<MODE>(loc, val, sLoc, sVal, sWarp);
 }
 
@@ -1252,10 +1254,10 @@ __device__ __forceinline__ void adj_vel_terms(DXP dxpT, DZP dzpT, float t4c, flo
     }
 }
 
-template <int MODE>
+template <int MODE, int ROWS>
 __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV ? 3 : 2)
     adjoint_kernel(const __grid_constant__ AdjArgs a, const __grid_constant__ AdjMaps m) {
-    using T = AdjTile<MODE>;
+    using T = AdjTile<MODE, ROWS>;
     using F = Fields<MODE>;
     constexpr int TX = T::TX, TZ = T::TZ, SX = T::SX, SZ = T::SZ, RVZ = T::RVZ, FS = T::FS, FV = T::FV;
     constexpr int NS = F::NS, NV = F::NV, NL = T::NL, NK = T::NK, NE = T::NE, RPW = TX / (kThreads / 32);
@@ -1335,7 +1337,7 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
     float nx_val[F::NINJ];
     auto prefetch_entries = [&](int shot) {
         const int q0 = a.inj_ptr ? a.inj_ptr[shot] : 0, q1 = a.inj_ptr ? a.inj_ptr[shot + 1] : 0;
-        if (q1 - q0 <= kThreads) adj_fetch<MODE>(a, q0, q1, x0, z0, nx_loc, nx_val);
+        if (q1 - q0 <= kThreads) adj_fetch<MODE, ROWS>(a, q0, q1, x0, z0, nx_loc, nx_val);
     };
     if (crank < nshots) prefetch_entries(crank);
     int i = 0;
@@ -1425,7 +1427,7 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
         if (!single) {
             for (int base = p0; base < p1; base += kThreads) {
                 __syncthreads();
-                const int n = adj_collect<MODE>(a, base, p1, x0, z0, sLoc, sVal, sWarp);
+                const int n = adj_collect<MODE, ROWS>(a, base, p1, x0, z0, sLoc, sVal, sWarp);
                 __syncthreads();
                 adj_apply<F::NINJ, FV>(sV, n, sLoc, sVal, dt);
             }
@@ -2084,9 +2086,9 @@ AdjPlan *make_adj_plan() { return new (std::nothrow) AdjPlan(); }
 void free_adj_plan(AdjPlan *p) { delete p; }
 
 // Tensor maps of one transposed step.
-template <int MODE>
+template <int MODE, int ROWS>
 static int adjoint_maps(const fwi_batch *b, long long slot0, int nseg, AdjMaps &m) {
-    using T = AdjTile<MODE>;
+    using T = AdjTile<MODE, ROWS>;
     using F = Fields<MODE>;
     const int cur = b->cur, nx = b->nx, pitch = b->pitch, ns = b->nshots;
     const long long field = (long long)ns * nx * pitch;
@@ -2101,44 +2103,76 @@ static int adjoint_maps(const fwi_batch *b, long long slot0, int nseg, AdjMaps &
     return rc;
 }
 
+static int sm_count() {
+    static std::atomic<int> known{0};
+    int n = known.load(std::memory_order_relaxed);
+    if (!n) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+            n = 148;
+        known.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // Shots processed side by side per tile (the cluster size, portable limit
 // 8): every CTA pays one cluster reduction, so the fewest CTAs that still
 // give about 2.5 waves of the resident-CTA slots (measured on 512 x 512 x 32
 // shots: 4 beats 2, 8 and 16).
 static int adjoint_cluster(int nshots, long long tiles, int ctas_per_sm) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-            sms = 148;
-    }
+    const int sms = sm_count();
     int c = 8;
     while (c > 1 && tiles * c * 2 > 5ll * sms * ctas_per_sm) c /= 2;
     return c < nshots ? c : nshots;
 }
 
+constexpr int adjoint_ctas(int mode) { return mode == FWI_SH ? 4 : mode == FWI_PSV ? 3 : 2; }  // per SM
+
+// Rows of the transposed step's tiles: 8, 16 or 32 (by 32 columns), or 64 for
+// the P-SV tile of 32 x 64.  A step cannot be shorter than one tile's chain of
+// phases, which is shorter for a smaller tile, so the smallest tile is taken
+// whose CTAs are resident all at once (8 rows: two per SM); with more CTAs
+// than that the largest tile, which repeats the least halo.  Measured, us a
+// step with tiles of 8 | 16 | 32 | 32 x 64: P-SV 128 x 96, 4 shots 7.2 | 7.3 |
+// 9.3 | 11.9; 183 x 270, 3 shots 12.9 | 9.3 | 11.4 | 12.7; 256 x 128, 16 shots
+// 20.6 | 20.6 | 16.5 | 18.1; 256 x 256, 8 shots 20.1 | 21.9 | 18.7 | 12.7.  SH
+// 64 x 64, 2 shots 6.2 | 6.8 | 8.8; 256 x 256, 4 shots 12.8 | 8.3 | 8.8, 16
+// shots 26.1 | 21.0 | 16.2.  Spin 64 x 64, 2 shots 8.3 | 10.4; 320 x 208, 4
+// shots 22.6 | 20.5.
 template <int MODE>
+static int adjoint_rows(const fwi_batch *b) {
+    constexpr int most = MODE == FWI_SPIN ? 16 : 32;
+    const int sms = sm_count();
+    for (int rows = 8; rows <= most; rows *= 2) {
+        const long long tiles = (long long)((b->nz + 31) / 32) * ((b->nx + rows - 1) / rows);
+        const int per_sm = rows == 8 ? 2 : adjoint_ctas(MODE);
+        if (tiles * adjoint_cluster(b->nshots, tiles, adjoint_ctas(MODE)) <= (long long)per_sm * sms) return rows;
+    }
+    return MODE == FWI_PSV ? 64 : most;
+}
+
+template <int MODE, int ROWS>
 static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPlan *plan, cudaStream_t st) {
-    using T = AdjTile<MODE>;
+    using T = AdjTile<MODE, ROWS>;
     static bool set = false;
     if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(adjoint_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(adjoint_kernel<MODE, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)T::bytes);
         if (e != cudaSuccess) return set_error(FWI_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         set = true;
     }
     AdjMaps &m = plan->maps[b->cur];
     if (a.slot < 0) {  // more stored shots than a map's coordinate counts: maps of this step's alone
-        const int rc = adjoint_maps<MODE>(b, a.it - b->seg0, 1, m);
+        const int rc = adjoint_maps<MODE, ROWS>(b, a.it - b->seg0, 1, m);
         if (rc) return rc;
     } else if (!plan->have[b->cur]) {
-        const int rc = adjoint_maps<MODE>(b, 0, b->nseg, m);
+        const int rc = adjoint_maps<MODE, ROWS>(b, 0, b->nseg, m);
         if (rc) return rc;
         plan->have[b->cur] = true;
     }
     const int C = adjoint_cluster(b->nshots, (long long)((b->nz + T::TZ - 1) / T::TZ) * ((b->nx + T::TX - 1) / T::TX),
-                                  MODE == FWI_SH ? 4 : MODE == FWI_PSV ? 3 : 2);
+                                  adjoint_ctas(MODE));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((b->nz + T::TZ - 1) / T::TZ, (b->nx + T::TX - 1) / T::TX, C);
     cfg.blockDim = dim3(kThreads, 1, 1);
@@ -2152,7 +2186,7 @@ static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPla
     set_pdl_attr(attr[1], true);
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, adjoint_kernel<MODE>, a, m);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, adjoint_kernel<MODE, ROWS>, a, m);
     if (e != cudaSuccess) return set_error(FWI_ECUDA, "adjoint_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("adjoint_kernel");
 }
@@ -2244,9 +2278,22 @@ int launch_adjoint_step(const fwi_batch *b, int it, bool pdl, AdjPlan *plan, cud
     a.g[0] = mode == FWI_SH ? b->stf[1] : b->stf[0];
     a.g[1] = mode == FWI_SH ? nullptr : b->stf[2];
     switch (mode) {
-        case FWI_SH: return launch_adjoint<FWI_SH>(b, a, pdl, plan, st);
-        case FWI_PSV: return b->adj_tile == 1 ? launch_adjoint<FWI_PSV>(b, a, pdl, plan, st) : launch_adjoint_wide(b, a, pdl, plan, st);
-        default: return launch_adjoint<FWI_SPIN>(b, a, pdl, plan, st);
+        case FWI_SH:
+            switch (adjoint_rows<FWI_SH>(b)) {
+                case 8: return launch_adjoint<FWI_SH, 8>(b, a, pdl, plan, st);
+                case 16: return launch_adjoint<FWI_SH, 16>(b, a, pdl, plan, st);
+                default: return launch_adjoint<FWI_SH, 32>(b, a, pdl, plan, st);
+            }
+        case FWI_PSV:
+            switch (b->adj_tile == 1 ? 32 : adjoint_rows<FWI_PSV>(b)) {
+                case 8: return launch_adjoint<FWI_PSV, 8>(b, a, pdl, plan, st);
+                case 16: return launch_adjoint<FWI_PSV, 16>(b, a, pdl, plan, st);
+                case 32: return launch_adjoint<FWI_PSV, 32>(b, a, pdl, plan, st);
+                default: return launch_adjoint_wide(b, a, pdl, plan, st);
+            }
+        default:
+            if (adjoint_rows<FWI_SPIN>(b) == 8) return launch_adjoint<FWI_SPIN, 8>(b, a, pdl, plan, st);
+            return launch_adjoint<FWI_SPIN, 16>(b, a, pdl, plan, st);
     }
 }
 

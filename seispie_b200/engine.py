@@ -206,7 +206,7 @@ class ShotBatch:
         self.tile = int(tile)
         self.ring = 0  # staging-ring depth of the row-marching kernel (0 = automatic)
         self.ctas_per_sm = 0  # row-marching grid: resident CTAs per SM (0 = all that fit)
-        self.adj_tile = 0  # P-SV transposed step: 0 = 32 x 64 tiles, 1 = 32 x 32 tiles
+        self.adj_tile = 0  # P-SV transposed step: 0 = tiles by size, 1 = 32 x 32 tiles
         # programmatic dependent launch between the steps of one call (fwi_batch.step_overlap)
         self.step_overlap = 1
 
