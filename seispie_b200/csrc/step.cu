@@ -1271,7 +1271,11 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
     const int crank = (int)cluster.block_rank(), csize = (int)cluster.num_blocks();
 
     const int tid = threadIdx.x, lane = tid & 31, ix0 = (tid >> 5) * RPW;
-    const int z0 = blockIdx.x * TZ, x0 = blockIdx.y * TX;
+    // tiles of one depth follow each other, so that those with receivers, which
+    // take longer, start first rather than in every wave (SH 512 x 512, 32 shots
+    // 90.5 -> 85.7 us a step; the 32 x 64 tiles gain 0.7 % there and lose 2 % on
+    // 300 x 900, 7 shots, and go by z first)
+    const int x0 = blockIdx.x * TX, z0 = blockIdx.y * TZ;
     const int nx = a.nx, nz = a.nz, pitch = a.pitch, nshots = a.nshots;
     const int gz = z0 + lane, col = lane + 4;
     const bool zin = gz < nz;
@@ -2174,7 +2178,7 @@ static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPla
     const int C = adjoint_cluster(b->nshots, (long long)((b->nz + T::TZ - 1) / T::TZ) * ((b->nx + T::TX - 1) / T::TX),
                                   adjoint_ctas(MODE));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((b->nz + T::TZ - 1) / T::TZ, (b->nx + T::TX - 1) / T::TX, C);
+    cfg.gridDim = dim3((b->nx + T::TX - 1) / T::TX, (b->nz + T::TZ - 1) / T::TZ, C);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = T::bytes;
     cfg.stream = st;
