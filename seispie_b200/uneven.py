@@ -106,6 +106,7 @@ class UnevenBatch:
             ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
             self.groups[mode] = (sel, arr, ws)
         self.graph = None
+        self._side = None  # the second wave type's stream
 
     def prepare(self):
         for sel, arr, ws in self.groups.values():
@@ -117,10 +118,27 @@ class UnevenBatch:
             d.cur = 0
 
     def run(self):
-        s = engine.stream_handle(None)
-        for sel, arr, ws in self.groups.values():
-            ntmax = max(it[0].nt for it in sel)
-            check(self.lib.fwi_multi_run(arr, len(sel), ws.data_ptr(), 0, ntmax, s), "fwi_multi_run")
+        """Every step of every group: the first wave type on the current
+        stream and the second beside it on a stream of its own, so that the
+        last, partly filled wave of CTAs of one type's step is filled by the
+        other's (joined before this returns)."""
+        main = torch.cuda.current_stream()
+        try:
+            for k, (sel, arr, ws) in enumerate(self.groups.values()):
+                if k and self._side is None:
+                    self._side = torch.cuda.Stream()
+                stream = self._side if k else main
+                if k:
+                    stream.wait_event(start)
+                else:
+                    start = main.record_event()
+                with torch.cuda.stream(stream):
+                    ntmax = max(it[0].nt for it in sel)
+                    check(self.lib.fwi_multi_run(arr, len(sel), ws.data_ptr(), 0, ntmax, engine.stream_handle(None)),
+                          "fwi_multi_run")
+        finally:
+            if self._side is not None:
+                main.wait_stream(self._side)
         for inst, m, b, d in self.items:
             b.cur = d.cur
 
