@@ -120,6 +120,19 @@ def two_level_segments(nt: int, mode: int) -> tuple:
     return min(k1, nt), min(k2, nt)
 
 
+def _copy_state(dst, src) -> None:
+    """Copy the wavefields of a state to or from a checkpoint: small fields in
+    one launch (12 fields of spin 320 x 208, 4 shots: 22 against 113 us for a
+    copy each; 5 of P-SV 128 x 96, 4 shots: 16 against 48 us), large ones by a
+    copy each, which is faster from there on (5 fields of 34 MB 70 against 72
+    us, of 134 MB 280 against 219 us)."""
+    if src[0].numel() * src[0].element_size() <= 40 << 20:
+        torch._foreach_copy_(list(dst), list(src))
+    else:
+        for d, s in zip(dst, src):
+            d.copy_(s)
+
+
 class ExactAdjoint:
     """Forward with checkpoints, then exact backward, for one batch of shots.
 
@@ -232,8 +245,7 @@ class ExactAdjoint:
         g = self.model.grid
         self.illum = torch.zeros((g.nx, g.pitch), dtype=torch.float64, device=self.model.device)
         for s in range(self.nseg):
-            for q, t in enumerate(b.state_tensors()):
-                self.ckpt[s, q].copy_(t)
+            _copy_state(self.ckpt[s].unbind(0), b.state_tensors())
             for v in b.vel[b.cur]:
                 engine.energy_accumulate(v, self.illum)
             n = min(self.K, self.t0 - s * self.K)
@@ -305,21 +317,18 @@ class ExactAdjoint:
             adj.run_transposed(adesc, self.nt, self.tail)
         for s in reversed(range(self.nseg)):
             s0, n = s * self.K, min(self.K, self.t0 - s * self.K)
-            for q, t in enumerate(fwd.state_tensors()):
-                t.copy_(self.ckpt[s, q])
+            _copy_state(fwd.state_tensors(), self.ckpt[s].unbind(0))
             if self.levels == 1:
                 reverse(s0, n)
                 continue
             nsub = math.ceil(n / self.K2)
             fwd.set_segment(self.rdesc, [None] * 6, [None] * 3, 0, 0)
             for jj in range(nsub):  # sub-checkpoints of this segment
-                for q, t in enumerate(fwd.state_tensors()):
-                    self.ckpt2[jj, q].copy_(t)
+                _copy_state(self.ckpt2[jj].unbind(0), fwd.state_tensors())
                 if jj < nsub - 1:
                     fwd.run(self.rdesc, False, s0 + jj * self.K2, self.K2)
             for jj in reversed(range(nsub)):
-                for q, t in enumerate(fwd.state_tensors()):
-                    t.copy_(self.ckpt2[jj, q])
+                _copy_state(fwd.state_tensors(), self.ckpt2[jj].unbind(0))
                 reverse(s0 + jj * self.K2, min(self.K2, n - jj * self.K2))
         fwd.set_segment(self.rdesc, [None] * 6, [None] * 3, 0, 0)
         return tuple(k)
@@ -360,8 +369,7 @@ class ExactAdjoint:
             with torch.cuda.stream(side):
                 if freed[j] is not None:
                     side.wait_event(freed[j])
-                for q, t in enumerate(fwd.state_tensors()):
-                    t.copy_(self.ckpt[s, q])
+                _copy_state(fwd.state_tensors(), self.ckpt[s].unbind(0))
                 fwd.set_segment(self.rdesc, bufs[j][0], bufs[j][1], s0, n)
                 fwd.run(self.rdesc, False, s0, n)
                 ev = torch.cuda.Event()
