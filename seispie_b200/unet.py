@@ -14,6 +14,8 @@ input has 3 channels, packed into 16 for the tensor-core convolutions.
 from __future__ import annotations
 
 
+import math
+
 import numpy as np
 import torch
 
@@ -31,6 +33,7 @@ LAYERS = (
     ("d2a", 64, 32, 32), ("d2b", 32, 0, 32),
     ("d1a", 32, 16, 16), ("d1b", 16, 0, 16),
 )
+CHANNELS = {name: (c0, c1, co) for name, c0, c1, co in LAYERS}
 
 
 def _align8(n: int) -> int:
@@ -69,8 +72,12 @@ class UNet:
     # ------------------------------------------------------------ parameters
     def view(self, name: str, t: torch.Tensor | None = None) -> torch.Tensor:
         o, shape = self.offsets[name]
-        n = int(np.prod(shape))
-        return (self.w if t is None else t)[o:o + n].view(shape)
+        return (self.w if t is None else t)[o:o + math.prod(shape)].view(shape)
+
+    def _addr(self, name: str, t: torch.Tensor) -> int:
+        """Address of a parameter in a flat vector: a view costs the host 7 us
+        more, and a training pass passes 90 of them."""
+        return t.data_ptr() + self.offsets[name][0] * t.element_size()
 
     def init_weights(self, seed: int) -> None:
         """He-normal 3x3 weights (fan-in 9 x real input channels), zero biases,
@@ -118,11 +125,11 @@ class UNet:
     def _act(self, n, h, w, c):
         return torch.empty((n, h, w, c), dtype=torch.bfloat16, device=self.device)
 
-    def _conv(self, name, x0, x1, out, n, h, w, relu=True):
-        _, c0, c1, co = next(L for L in LAYERS if L[0] == name)
-        check(self.lib.fwi_unet_conv3x3(ptr(x0), c0, ptr(x1), c1, ptr(self.view(name + ".w", self.wb)),
-                                        ptr(self.view(name + ".b")), co, ptr(out), co, None, 0, n, h, w, int(relu),
-                                        stream_handle(None)), "fwi_unet_conv3x3")
+    def _conv(self, name, x0, x1, out, n, h, w, st, relu=True):
+        c0, c1, co = CHANNELS[name]
+        check(self.lib.fwi_unet_conv3x3(ptr(x0), c0, ptr(x1), c1, self._addr(name + ".w", self.wb),
+                                        self._addr(name + ".b", self.w), co, ptr(out), co, None, 0, n, h, w, int(relu),
+                                        st), "fwi_unet_conv3x3")
         return out
 
     def forward(self, planes: torch.Tensor) -> torch.Tensor:
@@ -146,8 +153,8 @@ class UNet:
                 check(lib.fwi_unet_pool2(ptr(prev), ptr(p), CH[lvl - 1], n, 2 * hh, 2 * ww, st), "fwi_unet_pool2")
                 a["p%d" % lvl] = p
                 prev = p
-            ya = self._conv(name_a, prev, None, self._act(n, hh, ww, CH[lvl]), n, hh, ww)
-            yb = self._conv(name_b, ya, None, self._act(n, hh, ww, CH[lvl]), n, hh, ww)
+            ya = self._conv(name_a, prev, None, self._act(n, hh, ww, CH[lvl]), n, hh, ww, st)
+            yb = self._conv(name_b, ya, None, self._act(n, hh, ww, CH[lvl]), n, hh, ww, st)
             a[name_a], a[name_b] = ya, yb
             prev = yb
         for lvl, (name_a, name_b, skip) in zip((2, 1, 0), (("d3a", "d3b", "e3b"), ("d2a", "d2b", "e2b"),
@@ -156,35 +163,35 @@ class UNet:
             u = self._act(n, hh, ww, CH[lvl + 1])
             check(lib.fwi_unet_up2(ptr(prev), ptr(u), CH[lvl + 1], n, hh // 2, ww // 2, st), "fwi_unet_up2")
             a["u%d" % lvl] = u
-            ya = self._conv(name_a, u, a[skip], self._act(n, hh, ww, CH[lvl]), n, hh, ww)
-            yb = self._conv(name_b, ya, None, self._act(n, hh, ww, CH[lvl]), n, hh, ww)
+            ya = self._conv(name_a, u, a[skip], self._act(n, hh, ww, CH[lvl]), n, hh, ww, st)
+            yb = self._conv(name_b, ya, None, self._act(n, hh, ww, CH[lvl]), n, hh, ww, st)
             a[name_a], a[name_b] = ya, yb
             prev = yb
         out = torch.empty((n, h, w), dtype=torch.float32, device=self.device)
-        check(lib.fwi_unet_head(ptr(prev), ptr(self.view("head.w")), ptr(self.view("head.b")), ptr(out), n, h, w, st),
+        check(lib.fwi_unet_head(ptr(prev), self._addr("head.w", self.w), self._addr("head.b", self.w), ptr(out), n, h, w, st),
               "fwi_unet_head")
         self.acts, self.shape = a, (n, h, w)
         return out
 
-    def _conv_bwd(self, name, gy, x0, x1, n, h, w, need_input_grad=True, gx1=None):
+    def _conv_bwd(self, name, gy, x0, x1, n, h, w, st, need_input_grad=True, gx1=None):
         """Backward of one ReLU 3x3 layer given dL/d(output) gy (bf16,
         modified in place by the ReLU mask).  Writes the layer's weight and
         bias gradients into self.g; returns dL/d(in0) (and writes dL/d(in1)
         into gx1 when the layer has a skip input)."""
-        lib, st = self.lib, stream_handle(None)
-        _, c0, c1, co = next(L for L in LAYERS if L[0] == name)
+        lib = self.lib
+        c0, c1, co = CHANNELS[name]
         y = self.acts[name]
         check(lib.fwi_unet_relu_bwd(ptr(gy), ptr(y), gy.numel(), st), "fwi_unet_relu_bwd")
         need = lib.fwi_unet_wgrad_partials(co, c0 + c1, n, h, w)
         if self._part.numel() < need:
             self._part = torch.empty(need, dtype=torch.float32, device=self.device)
         check(lib.fwi_unet_conv3x3_wgrad(ptr(gy), co, ptr(x0), c0, ptr(x1), c1, n, h, w, ptr(self._part),
-                                         ptr(self.view(name + ".w", self.g)), ptr(self.view(name + ".b", self.g)), st),
+                                         self._addr(name + ".w", self.g), self._addr(name + ".b", self.g), st),
               "fwi_unet_conv3x3_wgrad")
         if not need_input_grad:
             return None
         wd = torch.empty(9 * co * (c0 + c1), dtype=torch.bfloat16, device=self.device)
-        check(lib.fwi_unet_flip_weights(ptr(self.view(name + ".w", self.wb)), ptr(wd), co, c0 + c1, st),
+        check(lib.fwi_unet_flip_weights(self._addr(name + ".w", self.wb), ptr(wd), co, c0 + c1, st),
               "fwi_unet_flip_weights")
         gx0 = self._act(n, h, w, c0)
         check(lib.fwi_unet_conv3x3(ptr(gy), co, None, 0, ptr(wd), None, c0 + c1, ptr(gx0), c0, ptr(gx1), c1, n, h, w,
@@ -200,8 +207,8 @@ class UNet:
         hs = [(h, w), (h // 2, w // 2), (h // 4, w // 4), (h // 8, w // 8)]
         g = self._act(n, h, w, 16)
         gout = gout.contiguous()
-        check(lib.fwi_unet_head_bwd(ptr(a["d1b"]), ptr(self.view("head.w")), ptr(gout), ptr(g),
-                                    ptr(self._part), ptr(self.g[self.offsets["head.w"][0]:]), n, h, w, st),
+        check(lib.fwi_unet_head_bwd(ptr(a["d1b"]), self._addr("head.w", self.w), ptr(gout), ptr(g),
+                                    ptr(self._part), self._addr("head.w", self.g), n, h, w, st),
               "fwi_unet_head_bwd")
         # head.w and head.b are adjacent in the flat vector only through the
         # 17-float result: copy the bias gradient to its slot
@@ -212,9 +219,9 @@ class UNet:
         for lvl, (name_a, name_b, skip) in zip((0, 1, 2), (("d1a", "d1b", "e1b"), ("d2a", "d2b", "e2b"),
                                                            ("d3a", "d3b", "e3b"))):
             hh, ww = hs[lvl]
-            g = self._conv_bwd(name_b, g, a[name_a], None, n, hh, ww)
+            g = self._conv_bwd(name_b, g, a[name_a], None, n, hh, ww, st)
             gskip = self._act(n, hh, ww, CH[lvl])
-            gu = self._conv_bwd(name_a, g, a["u%d" % lvl], a[skip], n, hh, ww, gx1=gskip)
+            gu = self._conv_bwd(name_a, g, a["u%d" % lvl], a[skip], n, hh, ww, st, gx1=gskip)
             skips[skip] = gskip
             g = self._act(n, hh // 2, ww // 2, CH[lvl + 1])
             check(lib.fwi_unet_up2_bwd(ptr(gu), ptr(g), CH[lvl + 1], n, hh // 2, ww // 2, st), "fwi_unet_up2_bwd")
@@ -226,8 +233,8 @@ class UNet:
                 gs = skips[name_b]
                 check(lib.fwi_unet_pool2_bwd(ptr(g), ptr(gs), CH[lvl], n, hh, ww, 1, st), "fwi_unet_pool2_bwd")
                 g = gs
-            g = self._conv_bwd(name_b, g, a[name_a], None, n, hh, ww)
-            g = self._conv_bwd(name_a, g, a[inp], None, n, hh, ww, need_input_grad=lvl > 0)
+            g = self._conv_bwd(name_b, g, a[name_a], None, n, hh, ww, st)
+            g = self._conv_bwd(name_a, g, a[inp], None, n, hh, ww, st, need_input_grad=lvl > 0)
 
     def adam(self, lr: float, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8) -> None:
         self.step += 1
