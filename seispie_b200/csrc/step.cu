@@ -134,6 +134,37 @@ __device__ __forceinline__ void stage_strided(float *dst, const float *const *sr
     }
 }
 
+// Add the n listed entries, times `scale`, to the staged components v (NINJ of
+// them, STRIDE apart; first warp).  32 entries in strictly increasing
+// locations, the usual case, are distinct cells and go in one pass; any other
+// 32 are summed one by one in entry order, since they may share a cell.  (One
+// thread adding every entry made the tiles with receivers the last to finish:
+// transposed P-SV step of 512 x 512, 32 shots 125 -> 116 us, of 256 x 128, 16
+// shots 19.6 -> 18.1 us; SH step with 200 receivers injected, 256 x 256, 4 shots
+// 8.7 -> 8.05 us, with 120 on 128 x 128, 2 shots 5.7 -> 4.6 us.)
+template <int NINJ, int STRIDE>
+__device__ __forceinline__ void add_entries(float *v, int n, const int *sLoc, const float *sVal, float scale) {
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    for (int base = 0; base < n; base += 32) {
+        const int q = base + lane;
+        const int loc = q < n ? sLoc[q] : 0x7fffffff - 32 + lane;
+        const int prev = __shfl_up_sync(0xffffffffu, loc, 1);
+        if (__all_sync(0xffffffffu, lane == 0 || loc > prev)) {
+            if (q < n) {
+#pragma unroll
+                for (int c = 0; c < NINJ; c++) v[c * STRIDE + loc] += scale * sVal[c * kThreads + q];
+            }
+        } else if (lane == 0) {
+            for (int r = base; r < min(base + 32, n); r++) {
+#pragma unroll
+                for (int c = 0; c < NINJ; c++) v[c * STRIDE + sLoc[r]] += scale * sVal[c * kThreads + r];
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // Entries of this shot at cells of the computed region, summed per cell in
 // entry order into J (NINJ components, VX x RVZ cells): the source scatter
 // stf_dsy / stf_dsxz (solver.py:78-93).  Returns whether any entry falls in
@@ -179,12 +210,7 @@ __device__ __forceinline__ bool scatter_entries(const int *inj_ptr, const int *i
             for (int c = 0; c < NINJ; c++) sVal[c * kThreads + pos] = val[c];
         }
         __syncthreads();
-        if (tid == 0) {
-            for (int q = 0; q < n_in; q++) {
-#pragma unroll
-                for (int c = 0; c < NINJ; c++) J[c * VX * RVZ + sLoc[q]] += sVal[c * kThreads + q];
-            }
-        }
+        add_entries<NINJ, VX * RVZ>(J, n_in, sLoc, sVal, 1.f);
         __syncthreads();
     }
     return has;
@@ -1148,7 +1174,7 @@ struct AdjTile {
 // velocity region add dt * u~ to the staged v~, summed per cell in entry
 // order.  adj_collect compacts up to kThreads entries [base, p1) into the
 // list (block-wide; the count it returns is block-uniform) and may run
-// while the staging copies are in flight; adj_apply adds them once v~ has
+// while the staging copies are in flight; add_entries adds them once v~ has
 // landed and the list is visible to the first warp.
 // adj_fetch: this thread's entry base + tid (its shared-memory location in
 // the staged v~, or -1, and its u~ values); no barrier, so it can be issued
@@ -1202,35 +1228,6 @@ __device__ __forceinline__ int adj_collect(const AdjArgs &a, int base, int p1, i
     float val[Fields<MODE>::NINJ];
     adj_fetch<MODE, ROWS>(a, base, p1, x0, z0, loc, val);
     return adj_compact<MODE>(loc, val, sLoc, sVal, sWarp);
-}
-
-// Add the n listed entries to the staged v~ (first warp).  32 entries in
-// strictly increasing locations, the usual case, are distinct cells and go in
-// one pass; any other 32 are summed one by one in entry order, since they may
-// share a cell.  (One thread adding every entry made the tiles with receivers
-// the last to finish: P-SV 512 x 512, 32 shots 125 -> 116 us a step, 256 x
-// 128, 16 shots 19.6 -> 18.1 us.)
-template <int NINJ, int FV>
-__device__ __forceinline__ void adj_apply(float *sV, int n, const int *sLoc, const float *sVal, float dt) {
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    for (int base = 0; base < n; base += 32) {
-        const int q = base + lane;
-        const int loc = q < n ? sLoc[q] : 0x7fffffff - 32 + lane;
-        const int prev = __shfl_up_sync(0xffffffffu, loc, 1);
-        if (__all_sync(0xffffffffu, lane == 0 || loc > prev)) {
-            if (q < n) {
-#pragma unroll
-                for (int c = 0; c < NINJ; c++) sV[c * FV + loc] += dt * sVal[c * kThreads + q];
-            }
-        } else if (lane == 0) {
-            for (int r = base; r < min(base + 32, n); r++) {
-#pragma unroll
-                for (int c = 0; c < NINJ; c++) sV[c * FV + sLoc[r]] += dt * sVal[c * kThreads + r];
-            }
-        }
-        __syncwarp();
-    }
 }
 
 // The velocity-like terms of the transposed step, (C^T t) per component,
@@ -1422,7 +1419,7 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
         }
         // v~ and the forward strain of this shot; u~ enters v~ (first warp)
         ok = mbar_wait(&bar[2], i & 1);
-        if (single && ok) adj_apply<F::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
+        if (single && ok) add_entries<F::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicExch(&g_device_status, 1);
             mbar_wait(&bar[2], i & 1);
@@ -1433,7 +1430,7 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
                 __syncthreads();
                 const int n = adj_collect<MODE, ROWS>(a, base, p1, x0, z0, sLoc, sVal, sWarp);
                 __syncthreads();
-                adj_apply<F::NINJ, FV>(sV, n, sLoc, sVal, dt);
+                add_entries<F::NINJ, FV>(sV, n, sLoc, sVal, dt);
             }
             __syncthreads();
         }
@@ -1829,7 +1826,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         // v~ of this shot; u~ enters v~ (first warp)
         ok = mbar_wait(&bar[2], i & 1);
-        if (single && ok) adj_apply<T::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
+        if (single && ok) add_entries<T::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicExch(&g_device_status, 1);
             mbar_wait(&bar[2], i & 1);
@@ -1843,7 +1840,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 wide_fetch(a, base, p1, x0, z0, loc, val);
                 const int n = adj_compact<FWI_PSV>(loc, val, sLoc, sVal, sWarp);
                 __syncthreads();
-                adj_apply<T::NINJ, FV>(sV, n, sLoc, sVal, dt);
+                add_entries<T::NINJ, FV>(sV, n, sLoc, sVal, dt);
             }
             __syncthreads();
         }

@@ -1,7 +1,7 @@
 """The transposed step's tiles of 8, 16, 32 rows and 32 x 64 cells, which the
 size of a batch selects: the adjoint fields of a shot have the same bits
-whichever tile computes them, and injected entries that share a cell or come
-in any order are all summed."""
+whichever tile computes them.  Entries injected into a transposed or a tiled
+step that share a cell or come in any order are all summed."""
 import numpy as np
 import pytest
 
@@ -119,3 +119,30 @@ def test_entries_sharing_cells_in_any_order(mode, nshots, n):
             np.add.at(mag, cells, dt * np.abs(vals[q, s * n:(s + 1) * n]).astype(np.float64))
             # FP32 sums of at most n terms, dt rounded to FP32, one product with the sponge
             assert np.all(np.abs(got[s] - sponge * want) <= (n + 3) * 2.0 ** -24 * mag)
+
+
+@pytest.mark.parametrize("mode", ["sh", "psv", "spin"])
+@pytest.mark.parametrize("n", [1, 33, 300])
+def test_sources_sharing_cells_in_any_order(mode, n):
+    """One tiled step from a zero state: v = sponge dt/rho sum(stf)."""
+    from seispie_b200.engine import ShotBatch
+    nx, nz, nshots = 70, 90, 2
+    rng = np.random.default_rng(n)
+    m = _model(mode, nx, nz, rng)
+    cells = rng.choice(rng.integers(0, nx * nz, 40), n).astype(np.int32)
+    vals = rng.standard_normal((2, nshots * n)).astype(np.float32)
+    b = ShotBatch(m, nshots, 1, np.array([5], np.int32), displacement=True)
+    stf = [None, None, None]
+    for q, c in enumerate(COMPS[mode][:2]):
+        stf[c] = torch.as_tensor(vals[q]).cuda()
+    inj = (np.arange(nshots + 1, dtype=np.int32) * n, np.tile(cells, nshots), np.arange(nshots * n, dtype=np.int32))
+    b.run(b.desc(inj=inj, stf=stf), False, 0, 1)
+    factor = (m.bound * m.buo).cpu().numpy()[:, :nz].reshape(-1).astype(np.float64)
+    for q, v in enumerate(b.vel[b.cur][:len(COMPS[mode][:2])]):
+        got = v.cpu().numpy()[..., :nz].reshape(nshots, -1)
+        for s in range(nshots):
+            want, mag = np.zeros(nx * nz), np.zeros(nx * nz)
+            np.add.at(want, cells, vals[q, s * n:(s + 1) * n].astype(np.float64))
+            np.add.at(mag, cells, np.abs(vals[q, s * n:(s + 1) * n]).astype(np.float64))
+            # FP32 sums of at most n terms and three products (one of them in `factor`)
+            assert np.all(np.abs(got[s] - factor * want) <= (n + 4) * 2.0 ** -24 * factor * mag)
