@@ -1133,7 +1133,11 @@ static int launch_march_any(MarchArgs &a, int nthr, int want, int cap, bool pdl,
 
 // ------------------------------------------------------------ resident steps
 
-constexpr int kResMinSteps = 24;  // fewer steps in one call are launched one by one
+// Fewer steps in one call are launched one by one: a resident call takes about
+// 13 us besides its steps, and from 8 steps on is still the faster (8 steps,
+// launched -> resident: SH 256 x 256, 1 shot 46.7 -> 32.4 us; P-SV 128 x 96, 4
+// shots 64.9 -> 35.3 us; 183 x 270, 3 shots 71.6 -> 52.8 us).
+constexpr int kResMinSteps = 8;
 
 // Clusters of csize CTAs of the resident kernel the GPU holds at once (0: none).
 template <int MODE, int I>
@@ -1224,6 +1228,8 @@ static double resident_us(int mode, int vel_rows, int stress_rows) {
     return 1.0 + 0.65 * (vel_rows + stress_rows) + spill;
 }
 
+constexpr double kResCallUs = 10.0;
+
 // The cluster size and rows per thread that finish a call first, or false
 // where launched steps do or a shot does not fit.
 struct ResidentPlan {
@@ -1231,10 +1237,11 @@ struct ResidentPlan {
     size_t bytes;
 };
 template <int MODE>
-static bool resident_plan(const fwi_batch *b, ResidentPlan *out) {
+static bool resident_plan(const fwi_batch *b, int nsteps, ResidentPlan *out) {
     const int groups = b->pitch / 4;
     if (groups > kResThreads) return false;
-    double best = 0.9 * launched_us(MODE, (double)b->nx * b->pitch * b->nshots);
+    // a call also loads and stores the state and finds the points
+    double best = 0.9 * launched_us(MODE, (double)b->nx * b->pitch * b->nshots) - kResCallUs / nsteps;
     bool found = false;
     for (int c = 1; c <= 16; c++) {
         const int rows = (b->nx + c - 1) / c;
@@ -1263,7 +1270,7 @@ int launch_resident(const fwi_batch *b, int it0, int nsteps, cudaStream_t st) {
     const bool seg = it0 + nsteps > b->seg0 && it0 < b->seg0 + b->nseg;
     if (nsteps < kResMinSteps || seg || b->ring || b->ctas_per_sm) return 1;
     ResidentPlan p;
-    if (!(mode == FWI_SH ? resident_plan<FWI_SH>(b, &p) : resident_plan<FWI_PSV>(b, &p))) return 1;
+    if (!(mode == FWI_SH ? resident_plan<FWI_SH>(b, nsteps, &p) : resident_plan<FWI_PSV>(b, nsteps, &p))) return 1;
     ResidentArgs a;
     a.nx = b->nx;
     a.nz = b->nz;

@@ -62,7 +62,7 @@ def _same(mode, ref, got):
 
 @pytest.mark.parametrize("mode", ["sh", "psv"])
 @pytest.mark.parametrize("nx,nz,nshots,steps", [
-    (3, 8, 1, 24), (5, 5, 2, 25), (7, 131, 3, 31), (48, 48, 1, 30), (50, 33, 5, 33), (61, 64, 40, 24),
+    (3, 8, 1, 8), (3, 8, 1, 24), (5, 5, 2, 25), (48, 60, 4, 9), (7, 131, 3, 31), (48, 48, 1, 30), (50, 33, 5, 33), (61, 64, 40, 24),
     (64, 64, 200, 25), (33, 512, 2, 24), (128, 96, 4, 40), (257, 100, 7, 26)])
 def test_resident_steps_bit_identical(mode, nx, nz, nshots, steps):
     ref, got, (tiled, resident) = _run(mode, nx, nz, nshots, [steps])
@@ -80,5 +80,5 @@ def test_resident_many_points(mode):
 @pytest.mark.parametrize("mode", ["sh", "psv"])
 def test_resident_and_launched_steps_mix(mode):
     """Short calls (launched steps) between long ones (resident)."""
-    ref, got, _ = _run(mode, 70, 90, 3, [25, 3, 30, 1, 24])
+    ref, got, _ = _run(mode, 70, 90, 3, [25, 3, 9, 30, 1, 8])
     _same(mode, ref, got)
