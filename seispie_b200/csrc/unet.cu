@@ -549,6 +549,7 @@ __global__ void __launch_bounds__(128, 4) wgrad_kernel(const bf16 *g, int cout, 
         }
     }
     const int r0 = lane >> 2, cq = (lane & 3) * 2;
+    const bool pair = ((uintptr_t)part & 7u) == 0;  // the caller's scratch may start at any float
 #pragma unroll
     for (int t = 0; t < 9; t++) {
         float *base = part + ((long long)blockIdx.x * 9 + t) * cout * ct;
@@ -557,9 +558,14 @@ __global__ void __launch_bounds__(128, 4) wgrad_kernel(const bf16 *g, int cout, 
             const int co = co0 + wm * 16 + r0 + half * 8;
 #pragma unroll
             for (int nb = 0; nb < 2; nb++) {
-                const int ci = ci0 + wn * 16 + nb * 8 + cq;
-                *reinterpret_cast<float2 *>(base + (long long)co * ct + ci) =
-                    make_float2(acc[t][nb][half * 2], acc[t][nb][half * 2 + 1]);
+                float *o = base + (long long)co * ct + ci0 + wn * 16 + nb * 8 + cq;
+                const float lo = acc[t][nb][half * 2], hi = acc[t][nb][half * 2 + 1];
+                if (pair) {
+                    *reinterpret_cast<float2 *>(o) = make_float2(lo, hi);
+                } else {
+                    o[0] = lo;
+                    o[1] = hi;
+                }
             }
         }
     }
