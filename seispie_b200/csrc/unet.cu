@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -515,20 +516,41 @@ __global__ void __launch_bounds__(128, 4) wgrad_kernel(const bf16 *g, int cout, 
         cp_async_commit();
         cp_async_wait_all();
         __syncthreads();
+        // 16 pixels of a tile row; EDGE: only the first `valid` of them lie in the image.  An outside pixel's
+        // gradient is staged as zero, but its neighbours in x may be pixels of the image, whose infinities and
+        // NaN a zero would not cancel: x is zeroed as well (in registers, the other taps read the same halo).
         const int j = lane >> 3;
-        for (int ks = kpart; ks < kWgTile / 16; ks += KS) {
-            const int r = ks * 16 / TW, c = ks * 16 % TW;
+        auto products = [&](int ks, int r, int c, int valid, auto edge_t) {
+            constexpr bool EDGE = decltype(edge_t)::value;
             uint32_t a[4];
             ldsm_x4_t(a, &sG[(ks * 16 + (j >> 1) * 8 + (lane & 7)) * GS + wm * 16 + (j & 1) * 8]);
+            // this lane's two pixels of either octet, low half first
+            const int k0 = (lane & 3) * 2;
+            auto keep = [&](int k) -> uint32_t {
+                return (k < valid ? 0x0000ffffu : 0u) | (k + 1 < valid ? 0xffff0000u : 0u);
+            };
+            const uint32_t m0 = keep(k0), m1 = keep(k0 + 8);
 #pragma unroll
             for (int t = 0; t < 9; t++) {
                 const int px = (r + t / 3) * (TW + 2) + c + t % 3;
                 uint32_t b[4];
                 ldsm_x4_t(b, &sX[(px + (j & 1) * 8 + (lane & 7)) * XS + wn * 16 + (j >> 1) * 8]);
+                if (EDGE) {
+                    b[0] &= m0;
+                    b[1] &= m1;
+                    b[2] &= m0;
+                    b[3] &= m1;
+                }
                 const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
                 mma16816(acc[t][0], a, b0);
                 mma16816(acc[t][1], a, b1);
             }
+        };
+        for (int ks = kpart; ks < kWgTile / 16; ks += KS) {
+            const int r = ks * 16 / TW, c = ks * 16 % TW;
+            const int valid = y0 + r < s.h ? s.w - (x0 + c) : 0;
+            if (valid >= 16) products(ks, r, c, 16, std::false_type{});
+            else if (valid > 0) products(ks, r, c, valid, std::true_type{});
         }
         __syncthreads();
     }

@@ -40,3 +40,34 @@ def test_scratch_at_any_float(n, h, w, c, co):
     for shift in (1, 2, 3):
         for a, b in zip(ref, _wgrad(x, g, shift)):
             assert torch.equal(a, b)
+
+
+def _reference(x, g):
+    """dw in 64 bits, summed over the pairs of pixels that both lie in the image and over no others."""
+    x, g = x.double(), g.double()
+    n, h, w, c = x.shape
+    dw = torch.zeros(9, g.shape[-1], c, dtype=torch.float64, device=x.device)
+    for t in range(9):
+        dy, dx = t // 3 - 1, t % 3 - 1
+        gy, gx = slice(max(0, -dy), min(h, h - dy)), slice(max(0, -dx), min(w, w - dx))
+        xy, xx = slice(max(0, dy), min(h, h + dy)), slice(max(0, dx), min(w, w + dx))
+        if h > abs(dy) and w > abs(dx):
+            a, b = g[:, gy, gx].reshape(-1, g.shape[-1]), x[:, xy, xx].reshape(-1, c)
+            dw[t] = (a[:, :, None] * b[:, None, :]).sum(0)
+    return dw
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (2, 9, 17), (1, 16, 16), (2, 10, 33), (1, 8, 40), (3, 4, 5)])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_values_beside_the_edges_meet_no_outside_pixel(n, h, w, value):
+    """A non-finite activation in the last row or column reaches the taps that
+    pair it with a gradient pixel of the image, and no other tap."""
+    for row, col in ((h - 1, 0), (0, w - 1), (h - 1, w - 1)):
+        x, g = _rand(n, h, w, 16, seed=3), _rand(n, h, w, 32, seed=4)
+        x[0, row, col, 5] = value
+        got, ref = _wgrad(x, g)[0].double(), _reference(x, g)
+        assert torch.equal(got.isnan(), ref.isnan())
+        assert torch.equal(got.isinf() * got.sign(), ref.isinf() * ref.sign())
+        ok = ref.isfinite()
+        # FP32 sums of exact products, as in the other weight-gradient tests
+        assert float((got - ref)[ok].norm()) <= 1e-5 * float(ref[ok].norm()) + 1e-30
