@@ -71,3 +71,19 @@ def test_values_beside_the_edges_meet_no_outside_pixel(n, h, w, value):
         ok = ref.isfinite()
         # FP32 sums of exact products, as in the other weight-gradient tests
         assert float((got - ref)[ok].norm()) <= 1e-5 * float(ref[ok].norm()) + 1e-30
+
+
+# one to eight images per tile, the last tile partly filled, one to more than eight partial sums per weight, 16- and
+# 32-column tiles
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (9, 1, 1), (700, 1, 1), (11, 2, 3), (150, 3, 4), (5, 7, 9), (2, 7, 16),
+                                   (3, 1, 20), (40, 3, 33), (3, 4, 33)])
+@pytest.mark.parametrize("c,co", [(16, 16), (32, 64)])
+def test_small_images(n, h, w, c, co):
+    x, g = _rand(n, h, w, c, seed=5), _rand(n, h, w, co, seed=6)
+    (dw, db), ref = _wgrad(x, g), _reference(x, g)
+    # sums of exact products in FP32: at most their number times 2^-24 of the sum of their sizes
+    size = _reference(x.abs(), g.abs())
+    assert bool(((dw.double() - ref).abs() <= n * h * w * 2.0 ** -24 * size).all())
+    assert float((dw.double() - ref).norm()) <= 1e-5 * float(ref.norm())
+    d = db.double() - g.double().sum((0, 1, 2))
+    assert bool((d.abs() <= n * h * w * 2.0 ** -24 * g.double().abs().sum((0, 1, 2))).all())
