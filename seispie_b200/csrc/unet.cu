@@ -1051,25 +1051,24 @@ int fwi::unet_device_status(int clear, int *status) {
 // over the channel tiles, at most kWgMaxTiles (2048 pixels in one FP32
 // accumulator).
 struct WgSplit {
-    int tw, tx, ty, pack, tiles, per, blocks;
+    int tw, tx, ty, pack, per;
+    long long tiles, blocks;
 };
+// any positive sizes
 static WgSplit wgrad_split(int cout, int ct, int n, int h, int w) {
     WgSplit p;
     p.tw = w > 16 ? 32 : 16;
     const int th = kWgTile / p.tw;
-    p.tx = (w + p.tw - 1) / p.tw;
-    p.ty = (h + th - 1) / th;
-    p.pack = (th + 1) / (h + 1);
+    p.tx = (w - 1) / p.tw + 1;
+    p.ty = (h - 1) / th + 1;
+    p.pack = h < th ? (th + 1) / (h + 1) : 1;
     if (p.pack > n) p.pack = n;
-    if (p.pack < 1) p.pack = 1;
-    const long long tiles = (long long)((n + p.pack - 1) / p.pack) * p.tx * p.ty;
-    const int chan = (cout / (cout % 32 == 0 ? 32 : 16)) * (ct / (ct % 32 == 0 ? 32 : 16));
-    const long long want = 592 / chan > 1 ? 592 / chan : 1;
-    long long per = (tiles + want - 1) / want;
-    if (per > kWgMaxTiles) per = kWgMaxTiles;
-    p.tiles = (int)tiles;
-    p.per = (int)per;
-    p.blocks = (int)((tiles + per - 1) / per);
+    p.tiles = (long long)((n - 1) / p.pack + 1) * p.tx * p.ty;
+    const long long chan = (long long)(cout / (cout % 32 == 0 ? 32 : 16)) * (ct / (ct % 32 == 0 ? 32 : 16));
+    const long long want = chan > 0 && chan < 592 ? 592 / chan : 1;
+    const long long per = (p.tiles - 1) / want + 1;
+    p.per = (int)(per < kWgMaxTiles ? per : kWgMaxTiles);
+    p.blocks = (p.tiles - 1) / p.per + 1;
     return p;
 }
 
@@ -1084,9 +1083,9 @@ static int launch_wgrad(const WgSplit &p, const bf16 *g, int cout, const bf16 *i
             return set_error(FWI_ECUDA, "unet_wgrad: shared-memory attribute refused");
         attr.store(true, std::memory_order_release);
     }
-    const dim3 grid(p.blocks, (cout / BMC) * ((c0 + c1) / BNC));
+    const dim3 grid((unsigned)p.blocks, (cout / BMC) * ((c0 + c1) / BNC));
     wgrad_kernel<BMC, BNC, TW, PACK><<<grid, 128, T::bytes, st>>>(g, cout, i0, c0, i1, c1, part, s, p.tx, p.ty, p.pack,
-                                                                  p.tiles, p.per);
+                                                                  (int)p.tiles, p.per);
     return check_launch("unet_wgrad");
 }
 
@@ -1169,6 +1168,7 @@ int fwi_unet_relu_bwd(void *g, const void *y, long long count, void *stream) {
 }
 
 long long fwi_unet_wgrad_partials(int cout, int cin, int n, int h, int w) {
+    if (cout <= 0 || cin <= 0 || n <= 0 || h <= 0 || w <= 0) return 0;
     const long long npix = (long long)n * h * w;
     const long long blocks = wgrad_split(cout, cin, n, h, w).blocks;
     const long long rblocks = (npix + kBiasPix - 1) / kBiasPix;
@@ -1190,7 +1190,7 @@ int fwi_unet_conv3x3_wgrad(const void *g, int cout, const void *in0, int c0, con
     const bf16 *gg = (const bf16 *)g, *i0 = (const bf16 *)in0, *i1 = (const bf16 *)in1;
     UREQ(npix / kWgTile < 0x7fffffffll / 64, "fwi_unet_conv3x3_wgrad: too many pixels");
     const WgSplit p = wgrad_split(cout, ct, n, h, wd);
-    const int nblk = p.blocks;
+    const int nblk = (int)p.blocks;
     const auto launch = p.tw == 32 ? (p.pack > 1 ? launch_wgrad_tw<32, true> : launch_wgrad_tw<32, false>)
                                    : (p.pack > 1 ? launch_wgrad_tw<16, true> : launch_wgrad_tw<16, false>);
     int rc = launch(p, gg, cout, i0, c0, i1, c1, part, s, st);
