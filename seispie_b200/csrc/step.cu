@@ -165,6 +165,18 @@ __device__ __forceinline__ void add_entries(float *v, int n, const int *sLoc, co
     }
 }
 
+// Wait (bounded) for the copies that `bar` counts, then add the entries if the
+// list is `whole`.  A wait that gives up does so for the warp: add_entries'
+// shuffles name every lane, and lanes that gave up alone would leave the others
+// waiting there for them.
+template <int NINJ, int STRIDE>
+__device__ __forceinline__ bool wait_and_add(uint64_t *bar, uint32_t parity, bool whole, float *v, int n,
+                                             const int *sLoc, const float *sVal, float scale) {
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+    if (whole && ok) add_entries<NINJ, STRIDE>(v, n, sLoc, sVal, scale);
+    return ok;
+}
+
 // Entries of this shot at cells of the computed region, summed per cell in
 // entry order into J (NINJ components, VX x RVZ cells): the source scatter
 // stf_dsy / stf_dsxz (solver.py:78-93).  Returns whether any entry falls in
@@ -1418,8 +1430,7 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
             }
         }
         // v~ and the forward strain of this shot; u~ enters v~ (first warp)
-        ok = mbar_wait(&bar[2], i & 1);
-        if (single && ok) add_entries<F::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
+        ok = wait_and_add<F::NINJ, FV>(&bar[2], i & 1, single, sV, n_in, sLoc, sVal, dt);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicExch(&g_device_status, 1);
             mbar_wait(&bar[2], i & 1);
@@ -1825,8 +1836,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             s4[2 * F4] = xz;
         }
         // v~ of this shot; u~ enters v~ (first warp)
-        ok = mbar_wait(&bar[2], i & 1);
-        if (single && ok) add_entries<T::NINJ, FV>(sV, n_in, sLoc, sVal, dt);
+        ok = wait_and_add<T::NINJ, FV>(&bar[2], i & 1, single, sV, n_in, sLoc, sVal, dt);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicExch(&g_device_status, 1);
             mbar_wait(&bar[2], i & 1);
