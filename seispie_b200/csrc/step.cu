@@ -561,10 +561,17 @@ template <int MODE, int TX, bool TMA>
 __global__ void __launch_bounds__(kThreads, MODE == FWI_SPIN ? 1 : 3)
     step_kernel_rw(const __grid_constant__ StepArgs a, const __grid_constant__ TmaMaps maps) {
     extern __shared__ __align__(128) float smem[];
+    // the previous step (the state this step reads, and the buffers it overwrites) is complete from here on.
+    // No grid_dep_trigger: the next step is launched as this one's last CTAs leave.  CTAs of the next step that
+    // come in earlier take the places that are free just then, unevenly over the SMs, which cost grids of about
+    // one wave more than the launch they hid: us a step serialised | triggered at the top | so: SH 320 x 208, 4
+    // shots, 500 receivers 6.2 | 8.0 | 4.9, 512 x 512, 1 shot 6.2 | 7.0 | 4.7, P-SV 256 x 256, 2 shots 6.2 | 6.9 |
+    // 4.8; over 207 grids in geometric mean 1 | 0.91 | 0.81.
+    grid_dep_wait();
     rw_body<MODE, TX, TMA>(a, maps, smem, blockIdx.y * TX, blockIdx.x * 32, blockIdx.z);
 }
 
-// Body of the register-window step for the tile (x0, z0) of `shot`.
+// Body of the register-window step for the tile (x0, z0) of `shot` (after grid_dep_wait).
 template <int MODE, int TX, bool TMA>
 __device__ __forceinline__ void rw_body(const StepArgs &a, const TmaMaps &maps, float *smem, int x0, int z0,
                                         int shot) {
@@ -577,10 +584,6 @@ __device__ __forceinline__ void rw_body(const StepArgs &a, const TmaMaps &maps, 
     const int nx = a.nx, nz = a.nz, pitch = a.pitch;
     const long long soff = (long long)shot * nx * pitch;
     bool has_inj;
-    // the next step may be scheduled; the previous one (the state this step reads, and the buffers it
-    // overwrites) is complete from here on
-    grid_dep_trigger();
-    grid_dep_wait();
     if constexpr (TMA) {
         const int r = prologue_tma<MODE, TX, TZ>(a, maps, sm, reinterpret_cast<uint64_t *>(smem + T::BAR_OFF), x0,
                                                  z0, shot);
@@ -684,7 +687,7 @@ struct MultiInst {
 
 template <int MODE, int TX>
 __global__ void __launch_bounds__(kThreads, MODE == FWI_SPIN ? 1 : 3)
-    step_kernel_multi(const MultiInst *inst, const int *prefix, int nactive, int it, int cur) {
+    step_kernel_multi(const MultiInst *inst, const int *prefix, int nactive, int it, int cur, int early) {
     extern __shared__ __align__(128) float smem[];
     __shared__ StepArgs sa;
     __shared__ int sinfo[4];
@@ -713,10 +716,26 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SPIN ? 1 : 3)
     if (threadIdx.x == 0) sa.it = it;
     __syncthreads();
     const TmaMaps &unused = *reinterpret_cast<const TmaMaps *>(inst);  // the cp.async body never reads it
+    // the previous step is complete from here on; the next one may be scheduled, but not two at once
+    grid_dep_wait();
+    if (early) grid_dep_trigger();
     rw_body<MODE, TX, false>(sa, unused, smem, sinfo[2], sinfo[3], sinfo[1]);
 }
 
 // ------------------------------------------------------------- launching
+
+static int sm_count() {
+    static std::atomic<int> known{0};
+    int n = known.load(std::memory_order_relaxed);
+    if (!n) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+            n = 148;
+        known.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
 
 struct TileShape {
     int tx, tz, rw;
@@ -1051,7 +1070,12 @@ static int launch_multi(const MultiInst *inst, const int *prefix, int nactive, i
     set_pdl_attr(attr[0], true);
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, step_kernel_multi<MODE, TX>, inst, prefix, nactive, it, cur);
+    // The next step may come in while this one runs, except where it makes the SMs unequal (as in
+    // step_kernel_rw): 1.5 to 3 CTAs per SM.  Relative to serialised launches, early | at the end: P-SV instances
+    // of 64-160 cells a side 99 CTAs 0.86 | 0.96, 263 CTAs 1.06 | 0.97, 558 CTAs 0.93 | 0.98, of 128-384 cells
+    // 2731 CTAs 0.99 | 1.02; SH and P-SV side by side, 16 batches in geometric mean 0.71 | 0.76 (at the top 0.77).
+    const int sms = sm_count(), early = blocks < sms * 3 / 2 || blocks > sms * 3;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, step_kernel_multi<MODE, TX>, inst, prefix, nactive, it, cur, early);
     if (e != cudaSuccess) return set_error(FWI_ECUDA, "step_kernel_multi launch: %s", cudaGetErrorString(e));
     return check_launch("step_kernel_multi");
 }
@@ -2112,19 +2136,6 @@ static int adjoint_maps(const fwi_batch *b, long long slot0, int nseg, AdjMaps &
     const float *vp[3] = {b->buo, b->bound, b->buo_j};
     for (int p = 0; p < T::NP && !rc; p++) rc = encode_map(&m.vp[p], vp[p], 2, pitch, nx, 1, T::SZ, T::VX);
     return rc;
-}
-
-static int sm_count() {
-    static std::atomic<int> known{0};
-    int n = known.load(std::memory_order_relaxed);
-    if (!n) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
-            n = 148;
-        known.store(n, std::memory_order_relaxed);
-    }
-    return n;
 }
 
 // Shots processed side by side per tile (the cluster size, portable limit
