@@ -88,10 +88,10 @@ static inline cudaError_t set_wait_limit_here(int polls) {
 // Programmatic dependent launch between consecutive steps of one time loop.
 // A step kernel launched with the ProgrammaticStreamSerialization attribute
 // may be scheduled while the previous step's kernel in the same stream is
-// still running: grid_dep_trigger (at the top of the row-marching and the
-// transposed step kernels) lets the next launch be scheduled once every CTA of
-// this grid has started, without it once every CTA has ended, and
-// grid_dep_wait blocks the calling thread until the previous grid has
+// still running: grid_dep_trigger (in the row-marching, the multi-instance and
+// the wide transposed step kernels) lets the next launch be scheduled once
+// every CTA of this grid has come to it, without it once every CTA has ended,
+// and grid_dep_wait blocks the calling thread until the previous grid has
 // completed with all its memory operations visible.  Every access to the
 // wavefields, the stores or the gradient comes after grid_dep_wait; only the
 // barrier set-up and loads of the model (which no step writes) may precede

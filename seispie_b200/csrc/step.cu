@@ -1340,7 +1340,6 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
 #pragma unroll
         for (int k = 0; k < NE; k++) tma_load_3d(sE + k * TX * TZ, &m.ef[k], z0, x0, (a.slot > 0 ? a.slot * nshots : 0) + shot, &bar[2]);
     };
-    grid_dep_trigger();
     if (tid == 0) {
 #pragma unroll
         for (int b = 0; b < 3; b++) mbar_init(&bar[b], 1);
@@ -1355,7 +1354,9 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
 #pragma unroll
         for (int p = 0; p < T::NP; p++) tma_load_2d(sP + p * FV, &m.vp[p], z0 - 4, x0 - 1, &bar[0]);
     }
-    // the previous step (adjoint state, gradient sums) is complete from here on
+    // the previous step (adjoint state, gradient sums) is complete from here on; as in step_kernel_rw the next one is
+    // not triggered early (362 batches in geometric mean 0.67 of their time without, 0.69 with a trigger here, 0.71
+    // with one at the top)
     grid_dep_wait();
     if (tid == 0 && crank < nshots) {
         issue_sig(crank);
