@@ -2155,22 +2155,28 @@ constexpr int adjoint_ctas(int mode) { return mode == FWI_SH ? 4 : mode == FWI_P
 // Rows of the transposed step's tiles: 8, 16 or 32 (by 32 columns), or 64 for
 // the P-SV tile of 32 x 64.  A step cannot be shorter than one tile's chain of
 // phases, which is shorter for a smaller tile, so the smallest tile is taken
-// whose CTAs are resident all at once (8 rows: two per SM); with more CTAs
-// than that the largest tile, which repeats the least halo.  Measured, us a
-// step with tiles of 8 | 16 | 32 | 32 x 64: P-SV 128 x 96, 4 shots 7.2 | 7.3 |
-// 9.3 | 11.9; 183 x 270, 3 shots 12.9 | 9.3 | 11.4 | 12.7; 256 x 128, 16 shots
-// 20.6 | 20.6 | 16.5 | 18.1; 256 x 256, 8 shots 20.1 | 21.9 | 18.7 | 12.7.  SH
-// 64 x 64, 2 shots 6.2 | 6.8 | 8.8; 256 x 256, 4 shots 12.8 | 8.3 | 8.8, 16
-// shots 26.1 | 21.0 | 16.2.  Spin 64 x 64, 2 shots 8.3 | 10.4; 320 x 208, 4
-// shots 22.6 | 20.5.
+// whose CTAs are resident at once and leave each other room; with more CTAs
+// the next larger one, which repeats less halo.  The limits, 1.75 to 3 CTAs
+// per SM, are where the larger tile becomes the faster in 90 batches of each
+// wave type.  Measured, us a step with tiles of 8 | 16 | 32 | 32 x 64: P-SV
+// 128 x 96, 4 shots 6.5 | 6.4 | 8.3 | 11.1; 183 x 270, 3 shots 13.2 | 9.2 |
+// 11.2 | 13.6; 282 x 91, 8 shots (432 CTAs of 16 rows) 14.2 | 13.9 | 10.2 |
+// 12.1; 256 x 128, 16 shots 20.4 | 20.2 | 14.2 | 18.3; 899 x 40, 7 shots (406
+// CTAs of 32 rows) 19.8 | 20.0 | 18.4 | 13.0; 256 x 256, 8 shots 20.3 | 21.9 |
+// 20.0 | 12.8.  SH 64 x 64, 2 shots 5.6 | 6.0 | 7.3; 256 x 256, 4 shots 12.8 |
+// 8.0 | 8.0; 300 x 300, 3 shots (570 CTAs of 16 rows) 15.1 | 12.4 | 10.1.
+// Spin 64 x 64, 2 shots 7.2 | 8.9; 136 x 42, 15 shots (272 CTAs of 8 rows) 18.1
+// | 13.1; 320 x 208, 4 shots 20.8 | 18.4.
 template <int MODE>
 static int adjoint_rows(const fwi_batch *b) {
     constexpr int most = MODE == FWI_SPIN ? 16 : 32;
     const int sms = sm_count();
     for (int rows = 8; rows <= most; rows *= 2) {
         const long long tiles = (long long)((b->nz + 31) / 32) * ((b->nx + rows - 1) / rows);
-        const int per_sm = rows == 8 ? 2 : adjoint_ctas(MODE);
-        if (tiles * adjoint_cluster(b->nshots, tiles, adjoint_ctas(MODE)) <= (long long)per_sm * sms) return rows;
+        // CTAs per SM up to which this tile is the faster, in quarters
+        constexpr int limit8 = MODE == FWI_SH ? 8 : MODE == FWI_PSV ? 10 : 7, limit = MODE == FWI_SH ? 12 : 10;
+        const long long ctas = tiles * adjoint_cluster(b->nshots, tiles, adjoint_ctas(MODE));
+        if (4 * ctas <= (long long)(rows == 8 ? limit8 : limit) * sms) return rows;
     }
     return MODE == FWI_PSV ? 64 : most;
 }
