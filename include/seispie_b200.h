@@ -240,9 +240,8 @@ int fwi_prepare_model(const float *rho, const float *j, const float *mu_c, const
  * record, and the injection entries of each shot sorted by cell (entries at
  * one cell keep their relative order, which fixes their summation order).
  * A call of 8 or more such steps on a grid whose shots fit the shared memory
- * of a cluster may run as one kernel (same bits): only the half of the
- * ping-pong pairs that `cur` selects afterwards is then written, while the
- * other keeps the state before the call or what it held. */
+ * of a cluster may run as one kernel (same bits, both halves of the ping-pong
+ * pairs as single steps leave them). */
 int fwi_run(fwi_batch *b, int adjoint, int it0, int nsteps, void *stream);
 
 /* Uneven batches: n independent forward batches of one mode (each with its

@@ -736,6 +736,7 @@ struct ResidentArgs {
     float *sig_out[3];
     const float *vel_in[2];
     float *vel_out[2];
+    float *sig_prev[3], *vel_prev[2];  // the other half: the state before the last step
     const float *buo, *bound;
     const float *ip[2];
     const int *inj_ptr, *inj_cell, *inj_row;
@@ -861,11 +862,26 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     }
     cluster.sync();
 
+    // the state of the own rows to global memory
+    auto store_state = [&](float *const(&sig)[3], float *const(&vel)[2]) {
+        for (int q = tid; q < n * a.groups; q += kResThreads) {
+            const int r = q / a.groups, c = 4 * (q - r * a.groups);
+            const long long g = soff + (long long)(row0 + r) * pitch + c;
+#pragma unroll
+            for (int f = 0; f < NS; f++) st4(sig[f] + g, ld4(S + f * FS + (r + 3) * RL + 4 + c));
+#pragma unroll
+            for (int c2 = 0; c2 < NV; c2++) st4(vel[c2] + g, ld4(V + c2 * FV + (r + 1) * RL + 4 + c));
+        }
+    };
     float *const up = rank > 0 ? cluster.map_shared_rank(S, rank - 1) : nullptr;
     float *const down = rank + 1 < C ? cluster.map_shared_rank(S, rank + 1) : nullptr;
     const int n_up = row0 - (rank > 0 ? (int)((long long)nx * (rank - 1) / C) : 0);  // rows of the CTA above
     for (int step = 0; step < a.nsteps; step++) {
         const int it = a.it0 + step, par = step & 1;
+        if (step + 1 == a.nsteps) {  // both halves end as the launched steps leave them
+            store_state(a.sig_prev, a.vel_prev);
+            __syncthreads();
+        }
         // stress row q of this step at this thread's columns
         auto srow = [&](int q) -> float * {
             int r = q;
@@ -998,15 +1014,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
         }
         cluster.sync();
     }
-    // ---- state back
-    for (int q = tid; q < n * a.groups; q += kResThreads) {
-        const int r = q / a.groups, c = 4 * (q - r * a.groups);
-        const long long g = soff + (long long)(row0 + r) * pitch + c;
-#pragma unroll
-        for (int f = 0; f < NS; f++) st4(a.sig_out[f] + g, ld4(S + f * FS + (r + 3) * RL + 4 + c));
-#pragma unroll
-        for (int c2 = 0; c2 < NV; c2++) st4(a.vel_out[c2] + g, ld4(V + c2 * FV + (r + 1) * RL + 4 + c));
-    }
+    store_state(a.sig_out, a.vel_out);
 }
 
 // Displacement traces from velocity traces: u(it) = u(it-1) + v(it) dt over
@@ -1263,7 +1271,7 @@ static bool resident_plan(const fwi_batch *b, int nsteps, ResidentPlan *out) {
 
 // All steps [it0, it0 + nsteps) of a displacement-free forward batch on the
 // resident kernel, the state going from half cur to the half that many
-// single steps would end in; 1 if the batch is left to launched steps.
+// single steps would end in, the state one step earlier to the other; 1 if the batch is left to launched steps.
 int launch_resident(const fwi_batch *b, int it0, int nsteps, cudaStream_t st) {
     const int mode = b->mode;
     // segment stores come from launched steps
@@ -1291,11 +1299,13 @@ int launch_resident(const fwi_batch *b, int it0, int nsteps, cudaStream_t st) {
     for (int f = 0; f < 3; f++) {
         a.sig_in[f] = f < ns ? b->sig[cur][f] : nullptr;
         a.sig_out[f] = f < ns ? b->sig[end][f] : nullptr;
+        a.sig_prev[f] = f < ns ? b->sig[1 - end][f] : nullptr;
     }
     for (int q = 0; q < 2; q++) {
         const bool on = q < nv;
         a.vel_in[q] = on ? b->vel[cur][q] : nullptr;
         a.vel_out[q] = on ? b->vel[end][q] : nullptr;
+        a.vel_prev[q] = on ? b->vel[1 - end][q] : nullptr;
         a.obs[q] = on ? b->obs[comp_slot_of(mode, q)] : nullptr;
     }
     a.buo = b->buo;
