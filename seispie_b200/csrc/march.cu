@@ -876,143 +876,146 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     float *const up = rank > 0 ? cluster.map_shared_rank(S, rank - 1) : nullptr;
     float *const down = rank + 1 < C ? cluster.map_shared_rank(S, rank + 1) : nullptr;
     const int n_up = row0 - (rank > 0 ? (int)((long long)nx * (rank - 1) / C) : 0);  // rows of the CTA above
-    for (int step = 0; step < a.nsteps; step++) {
-        const int it = a.it0 + step, par = step & 1;
-        if (step + 1 == a.nsteps) {  // both halves end as the launched steps leave them
-            store_state(a.sig_prev, a.vel_prev);
-            __syncthreads();
-        }
-        // stress row q of this step at this thread's columns
-        auto srow = [&](int q) -> float * {
-            int r = q;
-            if (par && q < 3) r = RM + 6 + q;
-            if (par && q >= n + 3) r = RM + 9 + q - n - 3;
-            return S + r * RL + 4 + j0;
-        };
-        // ---- velocity
-        if (nv > 0) {
-            Q4 w0[4], w1[4];  // D-x windows
+    // all steps but the last; then, once the state before it is in the other half (as launched steps leave it), the
+    // last.  Two loops, since a branch in the time loop costs every step 2-3 %.
+    for (int step = 0, end = a.nsteps - 1;; end++) {
+        for (; step < end; step++) {
+            const int it = a.it0 + step, par = step & 1;
+            // stress row q of this step at this thread's columns
+            auto srow = [&](int q) -> float * {
+                int r = q;
+                if (par && q < 3) r = RM + 6 + q;
+                if (par && q >= n + 3) r = RM + 9 + q - n - 3;
+                return S + r * RL + 4 + j0;
+            };
+            // ---- velocity
+            if (nv > 0) {
+                Q4 w0[4], w1[4];  // D-x windows
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const float *s = srow(v0 + k);
-                w0[k] = ld4(s + FX0 * FS);
-                if (NV > 1) w1[k] = ld4(s + FX1 * FS);
-            }
+                for (int k = 0; k < 3; k++) {
+                    const float *s = srow(v0 + k);
+                    w0[k] = ld4(s + FX0 * FS);
+                    if (NV > 1) w1[k] = ld4(s + FX1 * FS);
+                }
 #pragma unroll
-            for (int k = 0; k < I; k++) {
-                if (k < nv) {
-                    const int gr = row0 - 1 + v0 + k;
-                    const float *s = srow(v0 + k + 3), *sc = srow(v0 + k + 2);
-                    w0[(k + 3) & 3] = ld4(s + FX0 * FS);
-                    if (NV > 1) w1[(k + 3) & 3] = ld4(s + FX1 * FS);
-                    if (gr >= 0 && gr < nx) {
-                        const Q4 cz = ld4(sc + FZ * FS);
-                        Q4 ds[NV], vn[NV];
-                        if constexpr (MODE == FWI_SH) {
-                            ds[0] = keep4(dzm4(kz, sc + FZ * FS, cz), zm);
-                        } else {
-                            ds[0] = keep4(dzm4(kz, sc + FX1 * FS, w1[(k + 2) & 3]), zm);
-                            ds[NV - 1] = keep4(dzm4(kz, sc + FZ * FS, cz), zm);
-                        }
-                        if (gr >= 2 && gr < nx - 2) {
-                            ds[0] = add4(fdx(kx, w0[(k + 2) & 3], w0[(k + 1) & 3], w0[(k + 3) & 3], w0[k & 3]), ds[0]);
-                            if (NV > 1)
-                                ds[NV - 1] = add4(fdx(kx, w1[(k + 2) & 3], w1[(k + 1) & 3], w1[(k + 3) & 3], w1[k & 3]),
-                                                  ds[NV - 1]);
-                        }
-                        if (cnt[k] & 1) {  // sources, summed per cell in entry order (stf_dsy / stf_dsxz, solver.py:78-93)
-                            Q4 acc[NINJ];
+                for (int k = 0; k < I; k++) {
+                    if (k < nv) {
+                        const int gr = row0 - 1 + v0 + k;
+                        const float *s = srow(v0 + k + 3), *sc = srow(v0 + k + 2);
+                        w0[(k + 3) & 3] = ld4(s + FX0 * FS);
+                        if (NV > 1) w1[(k + 3) & 3] = ld4(s + FX1 * FS);
+                        if (gr >= 0 && gr < nx) {
+                            const Q4 cz = ld4(sc + FZ * FS);
+                            Q4 ds[NV], vn[NV];
+                            if constexpr (MODE == FWI_SH) {
+                                ds[0] = keep4(dzm4(kz, sc + FZ * FS, cz), zm);
+                            } else {
+                                ds[0] = keep4(dzm4(kz, sc + FX1 * FS, w1[(k + 2) & 3]), zm);
+                                ds[NV - 1] = keep4(dzm4(kz, sc + FZ * FS, cz), zm);
+                            }
+                            if (gr >= 2 && gr < nx - 2) {
+                                ds[0] = add4(fdx(kx, w0[(k + 2) & 3], w0[(k + 1) & 3], w0[(k + 3) & 3], w0[k & 3]), ds[0]);
+                                if (NV > 1)
+                                    ds[NV - 1] = add4(fdx(kx, w1[(k + 2) & 3], w1[(k + 1) & 3], w1[(k + 3) & 3], w1[k & 3]),
+                                                      ds[NV - 1]);
+                            }
+                            if (cnt[k] & 1) {  // sources, summed per cell in entry order (stf_dsy / stf_dsxz, solver.py:78-93)
+                                Q4 acc[NINJ];
 #pragma unroll
-                            for (int q = 0; q < NINJ; q++) acc[q] = zero4();
-                            const int base = gr * nz + j0, end = gr * nz + min(j0 + 4, nz);
-                            for (int e = inj_lo[k]; e < ih; e++) {
-                                const int at = e - il, cell = at < kResPts ? i_cell[at] : a.inj_cell[e];
-                                if (cell >= end) break;
+                                for (int q = 0; q < NINJ; q++) acc[q] = zero4();
+                                const int base = gr * nz + j0, end = gr * nz + min(j0 + 4, nz);
+                                for (int e = inj_lo[k]; e < ih; e++) {
+                                    const int at = e - il, cell = at < kResPts ? i_cell[at] : a.inj_cell[e];
+                                    if (cell >= end) break;
 #pragma unroll
-                                for (int q = 0; q < NINJ; q++) {
-                                    const float val = at < kResPts ? pts[((it & 1) * NINJ + q) * kResPts + at]
-                                                                   : a.stf[q][(long long)a.inj_row[e] * nt + it];
+                                    for (int q = 0; q < NINJ; q++) {
+                                        const float val = at < kResPts ? pts[((it & 1) * NINJ + q) * kResPts + at]
+                                                                       : a.stf[q][(long long)a.inj_row[e] * nt + it];
+#pragma unroll
+                                        for (int x = 0; x < 4; x++)
+                                            if (cell - base == x) elem(acc[q], x) += val;
+                                    }
+                                }
+#pragma unroll
+                                for (int q = 0; q < NV; q++) ds[q] = add4(ds[q], acc[q]);
+                            }
+#pragma unroll
+                            for (int c = 0; c < NV; c++) {
+                                float *v = V + c * FV + (v0 + k) * RL + 4 + j0;
+                                vn[c] = mul4(bnd[k], fma4(ds[c], buo[k], ld4(v)));
+                                st4(v, vn[c]);
+                            }
+                            if (cnt[k] & 2) {  // receivers record the new velocity (save_obs, solver.py:151-156)
+                                const int base = gr * nz + j0, end = gr * nz + min(j0 + 4, nz);
+                                for (int e = rec_lo[k]; e < rh; e++) {
+                                    const int at = e - rl, id = at < kResPts ? r_id[at] : a.rec_order[e];
+                                    const int cell = at < kResPts ? r_cell[at] : a.rec_cell[id];
+                                    if (cell >= end) break;
+                                    const long long o = ((long long)shot * a.nrec + id) * nt + it;
 #pragma unroll
                                     for (int x = 0; x < 4; x++)
-                                        if (cell - base == x) elem(acc[q], x) += val;
+                                        if (cell - base == x) {
+#pragma unroll
+                                            for (int q = 0; q < NV; q++)
+                                                if (a.obs[q]) a.obs[q][o] = elem(vn[q], x);
+                                        }
                                 }
                             }
-#pragma unroll
-                            for (int q = 0; q < NV; q++) ds[q] = add4(ds[q], acc[q]);
                         }
+                    }
+                }
+            }
+            __syncthreads();
+            if (step + 1 < a.nsteps) stage(it + 1);
+            // ---- stress
+            if (ns > 0) {
+                Q4 w[NV][4];  // velocity rows s-1 .. s+2
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+#pragma unroll
+                    for (int c = 0; c < NV; c++) w[c][k] = ld4(V + c * FV + (s0 + k) * RL + 4 + j0);
+#pragma unroll
+                for (int k = 0; k < I; k++) {
+                    if (k < ns) {
+                        const int gs = row0 + s0 + k;
+                        Q4 ex[NV], ez[NV];
 #pragma unroll
                         for (int c = 0; c < NV; c++) {
-                            float *v = V + c * FV + (v0 + k) * RL + 4 + j0;
-                            vn[c] = mul4(bnd[k], fma4(ds[c], buo[k], ld4(v)));
-                            st4(v, vn[c]);
+                            const float *v = V + c * FV + (s0 + k) * RL + 4 + j0;
+                            w[c][(k + 3) & 3] = ld4(v + 3 * RL);
+                            ez[c] = keep4(dzp4(kz, v + RL, w[c][(k + 1) & 3]), zp);
+                            if (gs >= 1 && gs < nx - 2) ex[c] = fdx(kx, w[c][(k + 2) & 3], w[c][(k + 1) & 3], w[c][(k + 3) & 3], w[c][k & 3]);
+                            else ex[c] = zero4();
                         }
-                        if (cnt[k] & 2) {  // receivers record the new velocity (save_obs, solver.py:151-156)
-                            const int base = gr * nz + j0, end = gr * nz + min(j0 + 4, nz);
-                            for (int e = rec_lo[k]; e < rh; e++) {
-                                const int at = e - rl, id = at < kResPts ? r_id[at] : a.rec_order[e];
-                                const int cell = at < kResPts ? r_cell[at] : a.rec_cell[id];
-                                if (cell >= end) break;
-                                const long long o = ((long long)shot * a.nrec + id) * nt + it;
+                        float *s = S + (s0 + k + 3) * RL + 4 + j0;
+                        Q4 o[NS];
+                        if constexpr (MODE == FWI_SH) {
+                            const Q4 dm = mul4(dt4, ip0[k]);
+                            o[0] = fma4(dm, ex[0], ld4(s));
+                            o[1] = fma4(dm, ez[0], ld4(s + FS));
+                        } else {
+                            const Q4 two{bc2(2.f), bc2(2.f)};
+                            const Q4 l2m = fma4(two, ip1[k], ip0[k]);
+                            o[0] = fma4(dt4, fma4(l2m, ex[0], mul4(ip0[k], ez[NV - 1])), ld4(s));
+                            o[1] = fma4(dt4, fma4(ip0[k], ex[0], mul4(l2m, ez[NV - 1])), ld4(s + FS));
+                            o[NS - 1] = fma4(dt4, mul4(ip1[k], add4(ez[0], ex[NV - 1])), ld4(s + (NS - 1) * FS));
+                        }
+                        const int q = s0 + k;
 #pragma unroll
-                                for (int x = 0; x < 4; x++)
-                                    if (cell - base == x) {
-#pragma unroll
-                                        for (int q = 0; q < NV; q++)
-                                            if (a.obs[q]) a.obs[q][o] = elem(vn[q], x);
-                                    }
-                            }
+                        for (int f = 0; f < NS; f++) {
+                            st4(s + f * FS, o[f]);
+                            // the neighbours' halo rows of the next step (even steps read the rows in place)
+                            if (up && q < 3) st4(up + f * FS + ((par ? n_up + 3 : RM + 9) + q) * RL + 4 + j0, o[f]);
+                            if (down && q >= n - 3) st4(down + f * FS + ((par ? 0 : RM + 6) + q - n + 3) * RL + 4 + j0, o[f]);
                         }
                     }
                 }
             }
+            cluster.sync();
         }
+        if (end == a.nsteps) break;
+        store_state(a.sig_prev, a.vel_prev);
         __syncthreads();
-        if (step + 1 < a.nsteps) stage(it + 1);
-        // ---- stress
-        if (ns > 0) {
-            Q4 w[NV][4];  // velocity rows s-1 .. s+2
-#pragma unroll
-            for (int k = 0; k < 3; k++)
-#pragma unroll
-                for (int c = 0; c < NV; c++) w[c][k] = ld4(V + c * FV + (s0 + k) * RL + 4 + j0);
-#pragma unroll
-            for (int k = 0; k < I; k++) {
-                if (k < ns) {
-                    const int gs = row0 + s0 + k;
-                    Q4 ex[NV], ez[NV];
-#pragma unroll
-                    for (int c = 0; c < NV; c++) {
-                        const float *v = V + c * FV + (s0 + k) * RL + 4 + j0;
-                        w[c][(k + 3) & 3] = ld4(v + 3 * RL);
-                        ez[c] = keep4(dzp4(kz, v + RL, w[c][(k + 1) & 3]), zp);
-                        if (gs >= 1 && gs < nx - 2) ex[c] = fdx(kx, w[c][(k + 2) & 3], w[c][(k + 1) & 3], w[c][(k + 3) & 3], w[c][k & 3]);
-                        else ex[c] = zero4();
-                    }
-                    float *s = S + (s0 + k + 3) * RL + 4 + j0;
-                    Q4 o[NS];
-                    if constexpr (MODE == FWI_SH) {
-                        const Q4 dm = mul4(dt4, ip0[k]);
-                        o[0] = fma4(dm, ex[0], ld4(s));
-                        o[1] = fma4(dm, ez[0], ld4(s + FS));
-                    } else {
-                        const Q4 two{bc2(2.f), bc2(2.f)};
-                        const Q4 l2m = fma4(two, ip1[k], ip0[k]);
-                        o[0] = fma4(dt4, fma4(l2m, ex[0], mul4(ip0[k], ez[NV - 1])), ld4(s));
-                        o[1] = fma4(dt4, fma4(ip0[k], ex[0], mul4(l2m, ez[NV - 1])), ld4(s + FS));
-                        o[NS - 1] = fma4(dt4, mul4(ip1[k], add4(ez[0], ex[NV - 1])), ld4(s + (NS - 1) * FS));
-                    }
-                    const int q = s0 + k;
-#pragma unroll
-                    for (int f = 0; f < NS; f++) {
-                        st4(s + f * FS, o[f]);
-                        // the neighbours' halo rows of the next step (even steps read the rows in place)
-                        if (up && q < 3) st4(up + f * FS + ((par ? n_up + 3 : RM + 9) + q) * RL + 4 + j0, o[f]);
-                        if (down && q >= n - 3) st4(down + f * FS + ((par ? 0 : RM + 6) + q - n + 3) * RL + 4 + j0, o[f]);
-                    }
-                }
-            }
-        }
-        cluster.sync();
     }
     store_state(a.sig_out, a.vel_out);
 }
