@@ -790,13 +790,14 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     const int v0 = seg * iv, nv = work ? min(iv, n + 3 - v0) : 0;
     const int s0 = seg * is, ns = work ? min(is, n - s0) : 0;
 
-    // ---- state into shared memory (zero outside the grid)
+    // ---- state into shared memory (zero outside the grid and in the padding columns, where it stays zero)
     for (int q = tid; q < (n + 6) * a.groups; q += kResThreads) {
         const int r = q / a.groups, c = 4 * (q - r * a.groups), gr = row0 - 3 + r;
         const bool in = gr >= 0 && gr < nx;
+        const bool cin[4] = {c < nz, c + 1 < nz, c + 2 < nz, c + 3 < nz};
 #pragma unroll
         for (int f = 0; f < NS; f++) {
-            const Q4 v = in ? ld4(a.sig_in[f] + soff + (long long)gr * pitch + c) : zero4();
+            const Q4 v = in ? keep4(ld4(a.sig_in[f] + soff + (long long)gr * pitch + c), cin) : zero4();
             st4(S + f * FS + r * RL + 4 + c, v);
             // the odd copies of halo rows outside the grid stay zero; the others are written by the first step
             if (r < 3) st4(S + f * FS + (RM + 6 + r) * RL + 4 + c, zero4());
@@ -805,7 +806,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
         if (r >= 2 && r < n + 5) {
 #pragma unroll
             for (int c2 = 0; c2 < NV; c2++)
-                st4(V + c2 * FV + (r - 2) * RL + 4 + c, in ? ld4(a.vel_in[c2] + soff + (long long)gr * pitch + c) : zero4());
+                st4(V + c2 * FV + (r - 2) * RL + 4 + c,
+                    in ? keep4(ld4(a.vel_in[c2] + soff + (long long)gr * pitch + c), cin) : zero4());
         }
     }
     // ---- model of this thread's cells (zero in the padding columns, which keeps them zero)

@@ -54,3 +54,18 @@ def test_both_halves(mode, nx, nz, nshots, chunks):
     for h in range(2):
         for x, y in zip(a.sig[h] + a.vel[h], b.sig[h] + b.vel[h]):
             assert torch.equal(x, y) and float(x.abs().max()) > 0
+
+
+@pytest.mark.parametrize("mode", ["sh", "psv"])
+@pytest.mark.parametrize("nx,nz,nshots", [(5, 6, 2), (50, 33, 3), (61, 131, 1)])
+@pytest.mark.parametrize("padding", [7.0, float("nan"), float("inf")])
+def test_row_padding(mode, nx, nz, nshots, padding):
+    """Whatever the rows' padding holds before the call, it is zero afterwards and no cell sees it."""
+    a, b = _run(mode, nx, nz, nshots, (9,), 3, padding), _run(mode, nx, nz, nshots, (9,), 0, padding)
+    clean = _run(mode, nx, nz, nshots, (9,), 0)
+    for h in range(2):
+        for x, y, z in zip(a.sig[h] + a.vel[h], b.sig[h] + b.vel[h], clean.sig[h] + clean.vel[h]):
+            assert torch.equal(y, x) and torch.equal(y, z)
+            assert float(y[..., nz:].abs().max()) == 0
+    for c in ((1,) if mode == "sh" else (0, 2)):
+        assert torch.equal(a.traces(c), b.traces(c))
