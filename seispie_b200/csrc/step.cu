@@ -1287,7 +1287,7 @@ __device__ __forceinline__ void adj_vel_terms(DXP dxpT, DZP dzpT, float t4c, flo
     }
 }
 
-template <int MODE, int ROWS>
+template <int MODE, int ROWS, bool ZFIRST>
 __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV ? 3 : 2)
     adjoint_kernel(const __grid_constant__ AdjArgs a, const __grid_constant__ AdjMaps m) {
     using T = AdjTile<MODE, ROWS>;
@@ -1307,8 +1307,9 @@ __global__ void __launch_bounds__(kThreads, MODE == FWI_SH ? 4 : MODE == FWI_PSV
     // tiles of one depth follow each other, so that those with receivers, which
     // take longer, start first rather than in every wave (SH 512 x 512, 32 shots
     // 90.5 -> 85.7 us a step; the 32 x 64 tiles gain 0.7 % there and lose 2 % on
-    // 300 x 900, 7 shots, and go by z first)
-    const int x0 = blockIdx.x * TX, z0 = blockIdx.y * TZ;
+    // 300 x 900, 7 shots, and go by z first).  ZFIRST: more tiles along z than the second extent of a launch grid
+    // holds (an instance of its own: a runtime choice here cost the other grids 1 %)
+    const int x0 = (ZFIRST ? blockIdx.y : blockIdx.x) * TX, z0 = (ZFIRST ? blockIdx.x : blockIdx.y) * TZ;
     const int nx = a.nx, nz = a.nz, pitch = a.pitch, nshots = a.nshots;
     const int gz = z0 + lane, col = lane + 4;
     const bool zin = gz < nz;
@@ -2181,12 +2182,15 @@ static int adjoint_rows(const fwi_batch *b) {
     return MODE == FWI_PSV ? 64 : most;
 }
 
-template <int MODE, int ROWS>
+template <int MODE, int ROWS, bool ZFIRST = false>
 static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPlan *plan, cudaStream_t st) {
     using T = AdjTile<MODE, ROWS>;
+    constexpr int kLarge = MODE == FWI_SPIN ? 16 : 32;  // the tile of every grid with that many
+    if constexpr (ROWS == kLarge && !ZFIRST)
+        if ((b->nz + T::TZ - 1) / T::TZ > 65535) return launch_adjoint<MODE, ROWS, true>(b, a, pdl, plan, st);
     static bool set = false;
     if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(adjoint_kernel<MODE, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(adjoint_kernel<MODE, ROWS, ZFIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)T::bytes);
         if (e != cudaSuccess) return set_error(FWI_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         set = true;
@@ -2203,7 +2207,8 @@ static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPla
     const int C = adjoint_cluster(b->nshots, (long long)((b->nz + T::TZ - 1) / T::TZ) * ((b->nx + T::TX - 1) / T::TX),
                                   adjoint_ctas(MODE));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((b->nx + T::TX - 1) / T::TX, (b->nz + T::TZ - 1) / T::TZ, C);
+    const int tx = (b->nx + T::TX - 1) / T::TX, tz = (b->nz + T::TZ - 1) / T::TZ;
+    cfg.gridDim = ZFIRST ? dim3(tz, tx, C) : dim3(tx, tz, C);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = T::bytes;
     cfg.stream = st;
@@ -2215,7 +2220,7 @@ static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPla
     set_pdl_attr(attr[1], true);
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, adjoint_kernel<MODE, ROWS>, a, m);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, adjoint_kernel<MODE, ROWS, ZFIRST>, a, m);
     if (e != cudaSuccess) return set_error(FWI_ECUDA, "adjoint_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("adjoint_kernel");
 }
