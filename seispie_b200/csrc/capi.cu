@@ -32,6 +32,14 @@ int check_launch(const char *what) {
     return 0;
 }
 
+// A launch call that returned an error: nothing was launched.  The runtime
+// keeps the error for the next check of the thread, which may belong to
+// another call, so it is taken out here.
+int launch_failed(const char *what, cudaError_t e) {
+    cudaGetLastError();
+    return set_error(FWI_ECUDA, "%s launch: %s", what, cudaGetErrorString(e));
+}
+
 // defined in step.cu / aux.cu
 struct StepPlan;  // tensor maps kept over a time loop
 StepPlan *make_step_plan();

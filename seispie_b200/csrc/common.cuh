@@ -155,6 +155,7 @@ inline EncodeTiledFn encode_fn() {
 // Error reporting shared by the C entry points (defined in capi.cu).
 int set_error(int code, const char *fmt, ...);
 int check_launch(const char *what);
+int launch_failed(const char *what, cudaError_t e);
 
 // Device-side status words of the kernels with bounded waits, read (and
 // optionally cleared) by fwi_device_status; each source file owns its own.

@@ -1130,7 +1130,7 @@ static int launch_march_mode(MarchArgs &a, int nthr, int want, int cap, bool pdl
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, march_kernel<MODE, WIDE, SEG>, a);
-    if (e != cudaSuccess) return set_error(FWI_ECUDA, "march_kernel launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return launch_failed("march_kernel", e);
     return check_launch("march_kernel");
 }
 
@@ -1207,7 +1207,7 @@ static int launch_resident_kernel(const ResidentArgs &a, int csize, int nshots, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, resident_kernel<MODE, I>, a);
-    if (e != cudaSuccess) return set_error(FWI_ECUDA, "resident_kernel launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return launch_failed("resident_kernel", e);
     return check_launch("resident_kernel");
 }
 

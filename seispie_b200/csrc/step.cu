@@ -827,7 +827,7 @@ static int launch_tile(const StepArgs &a, int nshots, int cur, bool pdl, StepPla
         cfg.attrs = attr;
         cfg.numAttrs = pdl ? 1 : 0;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, step_kernel_rw<MODE, TX, TMA>, a, maps);
-        if (e != cudaSuccess) return set_error(FWI_ECUDA, "step_kernel launch: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) return launch_failed("step_kernel", e);
     }
     return check_launch("step_kernel");
 }
@@ -1076,7 +1076,7 @@ static int launch_multi(const MultiInst *inst, const int *prefix, int nactive, i
     // 2731 CTAs 0.99 | 1.02; SH and P-SV side by side, 16 batches in geometric mean 0.71 | 0.76 (at the top 0.77).
     const int sms = sm_count(), early = blocks < sms * 3 / 2 || blocks > sms * 3;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, step_kernel_multi<MODE, TX>, inst, prefix, nactive, it, cur, early);
-    if (e != cudaSuccess) return set_error(FWI_ECUDA, "step_kernel_multi launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return launch_failed("step_kernel_multi", e);
     return check_launch("step_kernel_multi");
 }
 
@@ -2221,7 +2221,7 @@ static int launch_adjoint(const fwi_batch *b, const AdjArgs &a, bool pdl, AdjPla
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, adjoint_kernel<MODE, ROWS, ZFIRST>, a, m);
-    if (e != cudaSuccess) return set_error(FWI_ECUDA, "adjoint_kernel launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return launch_failed("adjoint_kernel", e);
     return check_launch("adjoint_kernel");
 }
 
@@ -2256,7 +2256,7 @@ static int launch_adjoint_wide(const fwi_batch *b, const AdjArgs &a, bool pdl, A
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, adjoint_wide_kernel, a, m);
-    if (e != cudaSuccess) return set_error(FWI_ECUDA, "adjoint_wide_kernel launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return launch_failed("adjoint_wide_kernel", e);
     return check_launch("adjoint_wide_kernel");
 }
 
