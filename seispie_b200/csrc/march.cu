@@ -1053,13 +1053,20 @@ bool march_supported(const fwi_batch *b) {
 
 constexpr size_t kMaxSmem = 227 * 1024;
 
+// The calling thread's device: a kernel's attributes and what fits at once are
+// kept per device.
+static int current_device() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : 0;
+}
+
 // Ring depth and resident CTAs per SM for a launch shape: the requested
 // depth, or the one with the most resident CTAs (shared memory and
-// registers both counted), the deepest among those.  Made once per shape;
-// the kernel's dynamic shared memory limit is the SM's throughout, so that a
-// shape's plan does not depend on which other shapes have run.
+// registers both counted), the deepest among those.  Made once per device and
+// shape; the kernel's dynamic shared memory limit is the SM's throughout, so
+// that a shape's plan does not depend on which other shapes have run.
 struct MarchPlan {
-    int nthr, rl, want, n, occ;
+    int dev, nthr, rl, want, n, occ;
     size_t bytes;
 };
 
@@ -1068,17 +1075,22 @@ static int march_choose(int nthr, int rl, int want, MarchPlan *out) {
     static std::mutex lock;
     static std::vector<MarchPlan> plans;
     const auto kernel = march_kernel<MODE, WIDE, SEG>;
+    const int dev = current_device();
     std::lock_guard<std::mutex> hold(lock);
-    if (plans.empty()) {
+    bool first = true;  // on this device
+    for (const MarchPlan &p : plans)
+        if (p.dev == dev) {
+            first = false;
+            if (p.nthr == nthr && p.rl == rl && p.want == want) {
+                *out = p;
+                return 0;
+            }
+        }
+    if (first) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
         if (e != cudaSuccess) return set_error(FWI_ECUDA, "march_kernel shared memory: %s", cudaGetErrorString(e));
     }
-    for (const MarchPlan &p : plans)
-        if (p.nthr == nthr && p.rl == rl && p.want == want) {
-            *out = p;
-            return 0;
-        }
-    MarchPlan best{nthr, rl, want, 0, 0, 0};
+    MarchPlan best{dev, nthr, rl, want, 0, 0, 0};
     for (int n : {3, 4, 6, 8}) {
         if (want && n != want) continue;
         const size_t b = march_bytes(MODE, rl, n);
@@ -1099,14 +1111,12 @@ static int march_choose(int nthr, int rl, int want, MarchPlan *out) {
 }
 
 static int sm_count() {
-    static std::atomic<int> sms{0};
-    int n = sms.load(std::memory_order_relaxed);
+    static std::atomic<int> sms[16];  // of the first devices, 0 until asked for
+    const int dev = current_device();
+    int n = dev < 16 ? sms[dev].load(std::memory_order_relaxed) : 0;
     if (!n) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
-            n = 148;
-        sms.store(n, std::memory_order_relaxed);
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+        if (dev < 16) sms[dev].store(n, std::memory_order_relaxed);
     }
     return n;
 }
@@ -1157,20 +1167,25 @@ template <int MODE, int I>
 static int resident_clusters(int csize, size_t bytes) {
     static std::mutex lock;
     struct Known {
-        int csize, clusters;
+        int dev, csize, clusters;
         size_t bytes;
     };
     static std::vector<Known> known;
+    const int dev = current_device();
     std::lock_guard<std::mutex> hold(lock);
     const auto kernel = resident_kernel<MODE, I>;
-    if (known.empty() &&
+    bool first = true;  // on this device
+    for (const Known &k : known)
+        if (k.dev == dev) {
+            first = false;
+            if (k.csize == csize && k.bytes == bytes) return k.clusters;
+        }
+    if (first &&
         (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess ||
          cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
         cudaGetLastError();
         return 0;
     }
-    for (const Known &k : known)
-        if (k.csize == csize && k.bytes == bytes) return k.clusters;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(csize, 1, 1);
@@ -1188,7 +1203,7 @@ static int resident_clusters(int csize, size_t bytes) {
         n = 0;
     }
     if (known.size() >= 1024) known.clear();
-    known.push_back(Known{csize, n, bytes});
+    known.push_back(Known{dev, csize, n, bytes});
     return n;
 }
 
