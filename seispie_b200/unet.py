@@ -60,6 +60,9 @@ class UNet:
         self.offsets["head.b"] = (off, (1,))
         off = _align8(off + 1)
         self.size = off
+        # elements that a pass reads or writes in each flat vector
+        last = self.offsets["head.b"][0] + 1
+        self.need = dict(w=last, g=last, wb=self.offsets[LAYERS[-1][0] + ".b"][0])
         dev = self.device
         self.w = torch.zeros(off, dtype=torch.float32, device=dev)
         self.wb = torch.zeros(off, dtype=torch.bfloat16, device=dev)
@@ -78,6 +81,16 @@ class UNet:
         """Address of a parameter in a flat vector: a view costs the host 7 us
         more, and a training pass passes 90 of them."""
         return t.data_ptr() + self.offsets[name][0] * t.element_size()
+
+    def _check_flat(self, *names: str) -> None:
+        """The flat vectors that a pass takes addresses in hold every
+        parameter (a view of a vector that was put in their place would
+        say so for each)."""
+        for k in names:
+            t = getattr(self, k)
+            if t.dim() != 1 or t.numel() < self.need[k]:
+                raise RuntimeError("UNet.%s: a flat vector of at least %d parameters is needed, not one of shape %s"
+                                   % (k, self.need[k], tuple(t.shape)))
 
     def init_weights(self, seed: int) -> None:
         """He-normal 3x3 weights (fan-in 9 x real input channels), zero biases,
@@ -138,6 +151,7 @@ class UNet:
         n, c, h, w = planes.shape
         if c != 3 or h % 8 or w % 8:
             raise ValueError("UNet input must be [n, 3, h, w] with h, w multiples of 8")
+        self._check_flat("w", "wb")
         lib, st = self.lib, stream_handle(None)
         a = {}
         x0 = self._act(n, h, w, 16)
@@ -200,6 +214,7 @@ class UNet:
 
     def backward(self, gout: torch.Tensor) -> None:
         """dL/d(output) [n, h, w] FP32 -> parameter gradients in self.g."""
+        self._check_flat("w", "wb", "g")
         lib, st = self.lib, stream_handle(None)
         n, h, w = self.shape
         a = self.acts
