@@ -69,3 +69,15 @@ def test_row_padding(mode, nx, nz, nshots, padding):
             assert float(y[..., nz:].abs().max()) == 0
     for c in ((1,) if mode == "sh" else (0, 2)):
         assert torch.equal(a.traces(c), b.traces(c))
+
+
+@pytest.mark.parametrize("mode", ["sh", "psv"])
+@pytest.mark.parametrize("nx,nz", [(40, 48), (9, 130)])
+def test_many_points(mode, nx, nz):
+    """More sources and receivers in a CTA's rows than it stages (64), by the launch count on resident steps."""
+    a, b = (_run(mode, nx, nz, 2, (27,), ring, npts=700) for ring in (3, 0))
+    for h in range(2):
+        for x, y in zip(a.sig[h] + a.vel[h], b.sig[h] + b.vel[h]):
+            assert torch.equal(x, y)
+    for c in ((1,) if mode == "sh" else (0, 2)):
+        assert torch.equal(a.traces(c), b.traces(c)) and float(a.traces(c).abs().max()) > 0
