@@ -135,9 +135,12 @@ typedef struct fwi_batch {
      * previous step is finishing, hiding launch latency and set-up; every
      * access to the state still waits for the previous step to complete, so
      * the results are bit-identical to 0, which serialises the launches.
-     * Worth it for a time loop that has the GPU to itself; a loop that shares
-     * the SMs with another stream's kernels runs faster with 0 (the early
-     * CTAs hold SM slots while they wait).  No counterpart in the reference
+     * Where the next step may come in early lies with each kernel (some let
+     * it in only as their last CTAs leave).  Worth it for a time loop that has
+     * the GPU to itself and for uneven groups side by side; the overlapped
+     * backward's recomputed and transposed steps, which fill the SMs together,
+     * run faster with 0 (early CTAs hold SM slots while they wait).
+     * fwi_multi_run goes by its first batch.  No counterpart in the reference
      * (its steps are separate Numba launches, solver.py:205-234). */
     int step_overlap;
 } fwi_batch;

@@ -29,11 +29,12 @@
 //     iteration ahead, outside the branches: a load inside one is waited for
 //     where the branches join.
 //   * What bounds it (P-SV 512 x 512, 32 shots): latency with 12 warps per SM
-//     (issue 44 %, DRAM 48 %), not the 470 MB a step has to move at 56 B per
-//     cell (72 us at the measured copy rate; the model and part of the state
-//     come from L2).  One row per barrier, scalar arithmetic and one thread
+//     (issue 45 %, 326 MB of DRAM traffic at 53 % of the device's nominal
+//     throughput), not the 336 MB that a step has to move, the state's 40 B
+//     per cell (51 us at the measured copy rate; the shots share the model,
+//     which L2 holds).  One row per barrier, scalar arithmetic and one thread
 //     issuing all copies: 88.7 us and 52.1 M warp instructions per step; this:
-//     69.7 us, 35 M.  1021 x 511, 64 shots: 284 -> 245 us (1.9 GB: 285 us at
+//     69.7 us, 34 M.  1021 x 511, 64 shots: 284 -> 245 us (1.34 GB: 204 us at
 //     the copy rate).  SH 512 x 512, 32 shots: 56 -> 41 us.  256 x 256, one SH
 //     shot: 11.2 -> 5.6 us, where the serial searches of the receiver list
 //     by one thread were most of the step (now a warp tests 32 places at once,
@@ -1156,10 +1157,10 @@ static int launch_march_any(MarchArgs &a, int nthr, int want, int cap, bool pdl,
 
 // ------------------------------------------------------------ resident steps
 
-// Fewer steps in one call are launched one by one: a resident call takes about
-// 13 us besides its steps, and from 8 steps on is still the faster (8 steps,
-// launched -> resident: SH 256 x 256, 1 shot 46.7 -> 32.4 us; P-SV 128 x 96, 4
-// shots 64.9 -> 35.3 us; 183 x 270, 3 shots 71.6 -> 52.8 us).
+// Fewer steps in one call are launched one by one: a resident call takes 9 to
+// 14 us more besides its steps than a launched one, and from 8 steps on is still
+// the faster (8 steps, launched -> resident: SH 256 x 256, 1 shot 48 -> 37 us;
+// P-SV 128 x 96, 4 shots 67 -> 39 us; 183 x 270, 3 shots 75 -> 58 us).
 constexpr int kResMinSteps = 8;
 
 // Clusters of csize CTAs of the resident kernel the GPU holds at once (0: none).
@@ -1256,7 +1257,7 @@ static double resident_us(int mode, int vel_rows, int stress_rows) {
     return 1.0 + 0.65 * (vel_rows + stress_rows) + spill;
 }
 
-constexpr double kResCallUs = 10.0;
+constexpr double kResCallUs = 10.0;  // of a call besides its steps, more than a launched call's (9 to 14 us)
 
 // The cluster size and rows per thread that finish a call first, or false
 // where launched steps do or a shot does not fit.

@@ -72,17 +72,9 @@ __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void *p) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(su32(p)));
 }
-__device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], const void *p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(su32(p)));
-}
 __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void *p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(su32(p)));
-}
-__device__ __forceinline__ void ldsm_x2_t(uint32_t (&r)[2], const void *p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-                 : "=r"(r[0]), "=r"(r[1])
                  : "r"(su32(p)));
 }
 // d += a (16x16, row-major) * b (16x8, column-major), bf16 inputs, f32 accumulators
