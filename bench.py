@@ -532,8 +532,9 @@ def main():
         steps = ev.get("steps", [])
         n_launch = sum(n for _, _, n in steps)
         per_launch_s = sum(e0.elapsed_time(e1) for e0, e1, _ in steps) * 1e-3 / max(1, n_launch)
-        # algorithmic bytes: stress (3) and velocity (2) read and written, lam, mu, dt/rho, sponge read
-        bytes_per_launch = nshots * nx * nz * (40 + 16)
+        # algorithmic bytes: stress (3) and velocity (2) of every shot read and written; lam, mu, dt/rho and sponge,
+        # which the shots share, read once
+        bytes_per_launch = nx * nz * (nshots * 40 + 16)
         kernel = "march_kernel<P-SV> (row-marching step, displacement-free; plain forward launches)"
         traffic_file = "march_kernel_psv_traffic.json"
         if not n_launch:  # every step in the stored tail (short runs): the forward sweep per step
