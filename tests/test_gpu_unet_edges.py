@@ -87,3 +87,28 @@ def test_small_images(n, h, w, c, co):
     assert float((dw.double() - ref).norm()) <= 1e-5 * float(ref.norm())
     d = db.double() - g.double().sum((0, 1, 2))
     assert bool((d.abs() <= n * h * w * 2.0 ** -24 * g.double().abs().sum((0, 1, 2))).all())
+
+
+@pytest.mark.parametrize("n,h,w,c", [(300, 2, 2, 8), (1, 70000, 2, 8), (2, 4, 66, 8), (1, 2, 6000, 24), (5, 6, 30, 16)])
+def test_rows_of_the_vector_maps(n, h, w, c):
+    """Rows shorter than, as long as and longer than a block, more rows than a launch grid: bit for bit against torch
+    in FP32 (one rounding of a product with 1/4, or of a sum of four values in the kernels' order)."""
+    from seispie_b200 import _lib
+    from seispie_b200.engine import check, ptr, stream_handle
+    lib, st = _lib.load(), stream_handle(None)
+    x, small, big = _rand(n, h, w, c, seed=7), _rand(n, h // 2, w // 2, c, seed=8), _rand(n, 2 * h, 2 * w, c, seed=9)
+
+    def four(t):
+        t = t.float()
+        return t[:, ::2, ::2] + t[:, ::2, 1::2] + t[:, 1::2, ::2] + t[:, 1::2, 1::2]
+
+    def run(name, src, shape, *more):
+        o = torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda")
+        check(getattr(lib, "fwi_unet_" + name)(ptr(src), ptr(o), c, n, h, w, *more, st), name)
+        return o
+
+    twice = lambda t: t.repeat_interleave(2, 1).repeat_interleave(2, 2)  # noqa: E731
+    assert torch.equal(run("pool2", x, small.shape), (0.25 * four(x)).bfloat16())
+    assert torch.equal(run("up2", x, big.shape), twice(x))
+    assert torch.equal(run("up2_bwd", big, x.shape), four(big).bfloat16())
+    assert torch.equal(run("pool2_bwd", small, x.shape, 0), (0.25 * twice(small.float())).bfloat16())
