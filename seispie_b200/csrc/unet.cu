@@ -29,7 +29,6 @@ namespace unet {
 
 using bf16 = __nv_bfloat16;
 
-constexpr int kConvStages = 5;  // staged slices of the mma.sync convolution
 constexpr int kAS = 24;   // shared row stride (bf16) of a 16-channel row: 48 bytes, conflict-free ldmatrix
 constexpr int kRedPix = 4096;  // pixels per head reduction block
 constexpr int kBiasPix = 512;  // pixels per bias-gradient block
@@ -101,16 +100,18 @@ __device__ __forceinline__ const bf16 *chan8(const bf16 *in0, int c0, const bf16
 //
 // The narrow levels of the network give few pixels, so the tile (BM pixels x
 // BN channels) is chosen to fill the chip, and the 9 * channels / 16 slices
-// stream through a ring of kConvStages stages with one barrier each: the
-// kernel is bound by the latency of that chain.  Neither changes the order in
-// which an output's products are summed.  Over the narrow layers of a
-// training step of eight 256 x 128 images: 28.3 -> 23.6 us on average.
-template <int BM, int BN>
+// stream through a ring of STAGES with one barrier each: the kernel is bound
+// by the latency of that chain where CTAs are few, and by how many of them an
+// SM holds, hence by the ring's shared memory, where they are many.  None of
+// the three changes the order in which an output's products are summed.  Over
+// the narrow layers of a training step of eight 256 x 128 images, five stages
+// for two: 28.3 -> 23.6 us on average.
+template <int BM, int BN, int STAGES>
 __global__ void __launch_bounds__(BM * 2) conv3x3_kernel(const bf16 *in0, int c0, const bf16 *in1, int c1, const bf16 *wt,
                                                          const float *bias, int cout, bf16 *out0, int d0, bf16 *out1,
                                                          int d1, Shape s, int relu) {
-    __shared__ __align__(128) bf16 sA[kConvStages][BM * kAS];
-    __shared__ __align__(128) bf16 sB[kConvStages][BN * kAS];
+    __shared__ __align__(128) bf16 sA[STAGES][BM * kAS];
+    __shared__ __align__(128) bf16 sB[STAGES][BN * kAS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long long hw = (long long)s.h * s.w, npix = s.n * hw;
     const long long p0 = (long long)blockIdx.x * BM;
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(BM * 2) conv3x3_kernel(const bf16 *in0, int c0
     }
     auto stage = [&](int kc) {
         if (kc < nk) {
-            const int tap = kc / nck, cc = (kc - tap * nck) * 16, buf = kc % kConvStages;
+            const int tap = kc / nck, cc = (kc - tap * nck) * 16, buf = kc % STAGES;
             const int dy = tap / 3 - 1, dx = tap % 3 - 1;
             const bf16 *src = aok ? chan8(in0, c0, in1, c1, s, an, ay + dy, ax + dx, cc + ahalf * 8) : nullptr;
             cp_async16(&sA[buf][apx * kAS + ahalf * 8], src ? src : in0, src ? 16 : 0);
@@ -144,12 +145,12 @@ __global__ void __launch_bounds__(BM * 2) conv3x3_kernel(const bf16 *in0, int c0
 #pragma unroll
     for (int nb = 0; nb < BN / 8; nb++) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.f;
 #pragma unroll
-    for (int kc = 0; kc < kConvStages - 1; kc++) stage(kc);
+    for (int kc = 0; kc < STAGES - 1; kc++) stage(kc);
     for (int kc = 0; kc < nk; kc++) {
-        cp_wait_slices<kConvStages - 2>();  // this thread's part of slice kc has landed
+        cp_wait_slices<STAGES - 2>();  // this thread's part of slice kc has landed
         __syncthreads();                    // everyone's has, and slice kc - 1 is consumed
-        stage(kc + kConvStages - 1);        // into the buffer of slice kc - 1
-        const int buf = kc % kConvStages;
+        stage(kc + STAGES - 1);        // into the buffer of slice kc - 1
+        const int buf = kc % STAGES;
         uint32_t a[4];
         ldsm_x4(a, &sA[buf][(warp * 16 + (lane & 15)) * kAS + (lane >> 4) * 8]);
 #pragma unroll
@@ -1124,21 +1125,32 @@ int fwi_unet_conv3x3(const void *in0, int c0, const void *in1, int c1, const voi
     bf16 *o0 = (bf16 *)out0, *o1 = (bf16 *)out1;
     if (g_conv_path == 0 && wd >= kTcMinWidth)
         return conv3x3_tc(i0, c0, i1, c1, wt, bias, cout, o0, d0, o1, d1, s, relu, st);
-    // the widest channel tile, unless it leaves SMs without a CTA: then 64 pixels, then fewer channels
-    // (4096 pixels x 128 channels: 64 x 32 tiles give 256 CTAs where 128 x 64 ones gave 64)
+    // The widest channel tile and 128 pixels, unless that gives too few CTAs: then 64 pixels, then fewer
+    // channels.  128 pixels are the faster from about one CTA per SM on, later where the channel tile is small
+    // and the chain long, sooner with 16 input channels (us, 128 pixels | 64: 64 -> 64 channels 102 CTAs 22.3 |
+    // 20.8, 128 CTAs 22.3 | 24.3, 256 CTAs 26.6 | 34.5; 96 -> 32 188 CTAs 31.7 | 28.3, 256 CTAs 32.4 | 33.0; 16 -> 16
+    // 47 CTAs 8.1 | 8.0, 102 CTAs 8.2 | 9.6).
     int bn = cout % 64 == 0 ? 64 : cout % 32 == 0 ? 32 : 16, bm = 128;
+    const int k = c0 + c1;
     auto ctas = [&] { return (npix + bm - 1) / bm * (cout / bn); };
-    if (ctas() < 296) bm = 64;
+    if (ctas() < (bn < 64 && k >= 48 ? 240 : bn == 16 && k == 16 ? 64 : 128)) bm = 64;
     if (bm == 64 && ctas() < 296 && bn == 64) bn = 32;
+    // Three stages where 128-pixel CTAs have long chains or are many, five elsewhere (us, five | three: 128 -> 48
+    // channels 768 CTAs 84 | 76, 128 -> 128 256 CTAs 48.6 | 46.5, 32 -> 32 128 CTAs 13.2 | 14.0, 782 CTAs 31.7 | 30.6,
+    // 16 -> 16 1563 CTAs 27.0 | 28.6).
+    const bool few = bm == 128 && (k >= 64 || (k >= 32 && ctas() >= 512));
     const dim3 grid((unsigned)((npix + bm - 1) / bm), cout / bn);
-#define CONV_LAUNCH(BM, BN) \
-    conv3x3_kernel<BM, BN><<<grid, BM * 2, 0, st>>>(i0, c0, i1, c1, wt, bias, cout, o0, d0, o1, d1, s, relu)
-    if (bm == 64 && bn == 64) CONV_LAUNCH(64, 64);
-    else if (bm == 64 && bn == 32) CONV_LAUNCH(64, 32);
-    else if (bm == 64) CONV_LAUNCH(64, 16);
-    else if (bn == 64) CONV_LAUNCH(128, 64);
-    else if (bn == 32) CONV_LAUNCH(128, 32);
-    else CONV_LAUNCH(128, 16);
+#define CONV_LAUNCH(BM, BN, STAGES) \
+    conv3x3_kernel<BM, BN, STAGES><<<grid, BM * 2, 0, st>>>(i0, c0, i1, c1, wt, bias, cout, o0, d0, o1, d1, s, relu)
+    if (bm == 64 && bn == 64) CONV_LAUNCH(64, 64, 5);
+    else if (bm == 64 && bn == 32) CONV_LAUNCH(64, 32, 5);
+    else if (bm == 64) CONV_LAUNCH(64, 16, 5);
+    else if (bn == 64 && few) CONV_LAUNCH(128, 64, 3);
+    else if (bn == 64) CONV_LAUNCH(128, 64, 5);
+    else if (bn == 32 && few) CONV_LAUNCH(128, 32, 3);
+    else if (bn == 32) CONV_LAUNCH(128, 32, 5);
+    else if (few) CONV_LAUNCH(128, 16, 3);
+    else CONV_LAUNCH(128, 16, 5);
 #undef CONV_LAUNCH
     return check_launch("unet_conv3x3");
 }

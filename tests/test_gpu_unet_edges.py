@@ -112,3 +112,26 @@ def test_rows_of_the_vector_maps(n, h, w, c):
     assert torch.equal(run("up2", x, big.shape), twice(x))
     assert torch.equal(run("up2_bwd", big, x.shape), four(big).bfloat16())
     assert torch.equal(run("pool2_bwd", small, x.shape, 0), (0.25 * twice(small.float())).bfloat16())
+
+
+# on 148 SMs: 64-pixel tiles by 16, 32 and 64 channels, 128-pixel tiles of three and of five stages by 16, 32 and 64
+# channels; images split over two inputs; fewer slices than stages is not possible (nine at least)
+@pytest.mark.parametrize("n,h,w,c0,c1,co", [
+    (1, 9, 7, 48, 0, 16), (3, 60, 61, 32, 0, 96), (5, 61, 43, 64, 0, 192), (9, 61, 63, 64, 0, 48), (17, 61, 63, 16, 0, 16),
+    (16, 61, 63, 64, 32, 32), (5, 61, 63, 32, 0, 32), (9, 61, 63, 64, 64, 64), (9, 61, 63, 16, 16, 64),
+    (40, 61, 63, 32, 0, 48)])
+def test_convolution_tiles_and_stages(n, h, w, c0, c1, co):
+    """Against torch in 64 bits: FP32 accumulation, one rounding to bf16 (2^-9 of the value) on output."""
+    import torch.nn.functional as F
+    from seispie_b200 import _lib
+    from seispie_b200.engine import check, ptr, stream_handle
+    lib, st, ct = _lib.load(), stream_handle(None), c0 + c1
+    x0, x1, wt = _rand(n, h, w, c0, seed=1), _rand(n, h, w, max(c1, 16), seed=2), _rand(9 * co * ct, seed=3)
+    b = torch.randn(co, device="cuda")
+    out = torch.full((n, h, w, co), float("nan"), dtype=torch.bfloat16, device="cuda")
+    check(lib.fwi_unet_conv3x3(ptr(x0), c0, ptr(x1) if c1 else None, c1, ptr(wt), ptr(b), co, ptr(out), co, None, 0, n,
+                               h, w, 0, st), "conv")
+    x = torch.cat([x0, x1[..., :c1]], -1).double().permute(0, 3, 1, 2)
+    ref = F.conv2d(x, wt.double().view(3, 3, co, ct).permute(2, 3, 0, 1), b.double(), padding=1).permute(0, 2, 3, 1)
+    scale = float(ref.abs().max())
+    assert bool(((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * scale).all())
